@@ -119,7 +119,7 @@ PFN_cuTensorMapEncodeTiled_v12000 get_encode() {
 }
 
 // ------------------------------------------------------------------ kernels
-__device__ __forceinline__ double ddiv_c(double x, double d, double inv_d, int pow2, uint64_t rw) {
+__device__ __forceinline__ double ddiv_c(double x, double d, double inv_d, int pow2, uint32_t rw) {
   return pow2 ? x * inv_d : fv_div_by(x, d, rw);
 }
 

@@ -58,11 +58,11 @@ struct DtArgs {
   int nblocks;
   double gamma, gm1, dx, dy, inv_dx, inv_dy;
   int dx_pow2, dy_pow2;
-  uint64_t rw_dx, rw_dy;  // reciprocal words of dx, dy (quotients when 1/dx is inexact)
+  uint32_t rw_dx, rw_dy;  // reciprocal words of dx, dy (quotients when 1/dx is inexact)
   double CFL, inv_tc, inv_visc;
 };
 
-__device__ __forceinline__ double div_spacing(double x, double d, double inv_d, int pow2, uint64_t rw) {
+__device__ __forceinline__ double div_spacing(double x, double d, double inv_d, int pow2, uint32_t rw) {
   return pow2 ? x * inv_d : fv2d::fv_div_by(x, d, rw);
 }
 

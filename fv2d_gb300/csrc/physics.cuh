@@ -58,15 +58,15 @@ __host__ __device__ __forceinline__ float fv_sqrt(float x) { return sqrtf(x); }
 // Several quotients by one divisor: r = fv_recip(b) once, fv_div_by(a, b, r)
 // per dividend (binary64 on the device: the reciprocal word of b is formed
 // once; the quotients are the same correctly rounded values as a / b).
-__host__ __device__ __forceinline__ uint64_t fv_recip(double b) {
+__host__ __device__ __forceinline__ uint32_t fv_recip(double b) {
 #ifdef __CUDA_ARCH__
   return softfp::recip_of(b);
 #else
   (void)b;
-  return 0ull;
+  return 0u;
 #endif
 }
-__host__ __device__ __forceinline__ double fv_div_by(double a, double b, uint64_t r) {
+__host__ __device__ __forceinline__ double fv_div_by(double a, double b, uint32_t r) {
 #ifdef __CUDA_ARCH__
   return softfp::div_by(a, b, r);
 #else
@@ -74,8 +74,8 @@ __host__ __device__ __forceinline__ double fv_div_by(double a, double b, uint64_
   return a / b;
 #endif
 }
-__host__ __device__ __forceinline__ uint64_t fv_recip(float) { return 0ull; }
-__host__ __device__ __forceinline__ float fv_div_by(float a, float b, uint64_t) { return a / b; }
+__host__ __device__ __forceinline__ uint32_t fv_recip(float) { return 0u; }
+__host__ __device__ __forceinline__ float fv_div_by(float a, float b, uint32_t) { return a / b; }
 
 // Comparisons, fmin / fmax and scalings by 1/2: on the device, binary64 goes
 // through the bit-pattern forms of softfp.cuh (IEEE results, integer pipe).
@@ -115,31 +115,49 @@ __host__ __device__ __forceinline__ float fv_mul(float x, float y) { return x * 
 __host__ __device__ __forceinline__ bool fv_isnan(float x) { return isnan(x); }
 
 // Products moved from the binary64 pipe to the integer pipes (softfp::mul_rn),
-// by group: the step is bound by the binary64 pipe, and moving every product
-// would make the integer pipes the bound instead.  FV2D_SOFT_MUL is a mask
-// (bit GROUP - 1 set: that group on the integer pipes); the groups are
-//   1  HLLC: energies, p gamma, u* numerator, mass and momentum fluxes
-//   2  HLLC: rho/2 (u^2 + v^2)
+// by group: a product holds the binary64 pipe for 64 cycles of an SM
+// sub-partition, an integer-pipe one the ALU for about as long, so the set
+// that balances the two is the fastest.  FV2D_SOFT_MUL is a mask (bit
+// GROUP - 1 set: that group on the integer pipes); the groups are
+//   1  HLLC: squared velocities, p gamma, u* numerator, fluxes
+//   2  HLLC: total energy (rho/2 (u^2 + v^2), p / (gamma - 1))
 //   3  the update's dt (F_L - F_R) products
 //   4  consToPrim: kinetic energy and (E - Ek)(gamma - 1)
 //   5  HLLC: rho (u - S)
 //   6  HLLC: p* numerator
-//   7  HLLC: star state
-//   8  HLLC: energy flux
+//   7  HLLC: star energy
+//   8  (unused)
 //   9  HLL: products of each side's state (kinetic energy, fluxes, momenta)
 //  10  HLL: the HLL average's products by the wave speeds
 //  11  viscous face terms
 //  12  conduction fluxes and the conduction / viscosity update products
 //  13  MUSCL-Hancock predictor
 //  14  FSLP
-// The default set measured fastest on the Sedov step.
+// Measured (ms per step; group on the binary64 pipe | on the integer pipes):
+// KH 2048^2 HLLC: 5 and 6 1.10 | 1.12, 7 1.10 | 1.13; Sedov 2048^2: 2 1.01 |
+// 0.99; FSLP RK2 777 x 1501: 14 0.372 | 0.358; RT 1024 x 3072: 12 1.68 | 1.64.
+// The viscous kernels also move group 10 (1.64 | 1.60); without viscosity it
+// is slower there (PCM-HLL 1000 x 600: 1.53 | 1.63 for five steps).
 #ifndef FV2D_SOFT_MUL
-#define FV2D_SOFT_MUL 4365
+#define FV2D_SOFT_MUL 14607
 #endif
 template <int GROUP, class R>
 __host__ __device__ __forceinline__ R mulx(R a, R b) {
   if constexpr ((FV2D_SOFT_MUL >> (GROUP - 1)) & 1) return fv_mul(a, b);
   else return a * b;
+}
+
+// {x0 y0, x1 y1} of one group: on the integer pipes in one call
+template <int GROUP>
+__device__ __forceinline__ void mulx2(double x0, double y0, double x1, double y1, double &r0, double &r1) {
+  if constexpr ((FV2D_SOFT_MUL >> (GROUP - 1)) & 1) {
+    const double2 r = softfp::mul2_rn(x0, y0, x1, y1);
+    r0 = r.x;
+    r1 = r.y;
+  } else {
+    r0 = x0 * y0;
+    r1 = x1 * y1;
+  }
 }
 
 enum { IR = 0, IU = 1, IV = 2, IP = 3, IE = 3 };
@@ -156,7 +174,7 @@ struct Gas {
   R gm1;     // gamma0 - 1.0
   R entho;   // 1.0 / (gamma0 - 1.0)               (RiemannSolvers.h:76)
   R fslp_K;  // FSLP K                              (SimInfo.h:399)
-  uint64_t rgm1;  // fv_recip(gm1): the divisions by gamma0 - 1 (set by make_gas)
+  uint32_t rgm1;  // fv_recip(gm1): the divisions by gamma0 - 1 (set by make_gas)
 };
 
 template <class R>
@@ -199,7 +217,7 @@ __device__ __forceinline__ R sound_speed(const S4<R> &q, const Gas<R> &g) {
 }
 // the same with the reciprocal of q.r already formed (fv_recip)
 template <class R>
-__device__ __forceinline__ R sound_speed_r(const S4<R> &q, const Gas<R> &g, uint64_t rr) {
+__device__ __forceinline__ R sound_speed_r(const S4<R> &q, const Gas<R> &g, uint32_t rr) {
   return dsqrt(fv_div_by(mulx<1>(q.p, g.gamma), q.r, rr));
 }
 
@@ -217,10 +235,10 @@ __device__ __forceinline__ R sel(bool c, R a, R b) {
 
 // RiemannSolvers.h:7-51.  All three candidates are evaluated, then selected
 // in the reference's branch order (SL >= 0, SR <= 0, else the HLL state).
-template <class R>
+template <bool SOFT_AVERAGE = false, class R>
 __device__ __forceinline__ void riemann_hll(const S4<R> &qL, const S4<R> &qR, S4<R> &f, R &pout, const Gas<R> &g) {
   // every quotient by rho_L (rho_R) shares one reciprocal
-  const uint64_t rL = fv_recip(qL.r), rR = fv_recip(qR.r);
+  const uint32_t rL = fv_recip(qL.r), rR = fv_recip(qR.r);
   const R aL = sound_speed_r(qL, g, rL);
   const R aR = sound_speed_r(qR, g, rR);
   const R sminL = qL.u - aL;
@@ -244,14 +262,15 @@ __device__ __forceinline__ void riemann_hll(const S4<R> &qL, const S4<R> &qR, S4
   const R mvL = mulx<9>(qL.r, qL.v), mvR = mulx<9>(qR.r, qR.v);
   const R uEL = (fv_div_by(fv_half(mulx<9>(ruL, ruL) + mulx<9>(mvL, mvL)), qL.r, rL) + peL);
   const R uER = (fv_div_by(fv_half(mulx<9>(ruR, ruR) + mulx<9>(mvR, mvR)), qR.r, rR) + peR);
-  const R SLSR = mulx<10>(SL, SR);
+  auto avg = [](R a, R b) { return SOFT_AVERAGE ? fv_mul(a, b) : mulx<10>(a, b); };
+  const R SLSR = avg(SL, SR);
   const R den = SR - SL;
-  const uint64_t rden = fv_recip(den);
+  const uint32_t rden = fv_recip(den);
   S4<R> FM;
-  FM.r = fv_div_by(mulx<10>(SR, FL.r) - mulx<10>(SL, FR.r) + mulx<10>(SLSR, qR.r - qL.r), den, rden);
-  FM.u = fv_div_by(mulx<10>(SR, FL.u) - mulx<10>(SL, FR.u) + mulx<10>(SLSR, ruR - ruL), den, rden);
-  FM.v = fv_div_by(mulx<10>(SR, FL.v) - mulx<10>(SL, FR.v) + mulx<10>(SLSR, mvR - mvL), den, rden);
-  FM.p = fv_div_by(mulx<10>(SR, FL.p) - mulx<10>(SL, FR.p) + mulx<10>(SLSR, uER - uEL), den, rden);
+  FM.r = fv_div_by(avg(SR, FL.r) - avg(SL, FR.r) + avg(SLSR, qR.r - qL.r), den, rden);
+  FM.u = fv_div_by(avg(SR, FL.u) - avg(SL, FR.u) + avg(SLSR, ruR - ruL), den, rden);
+  FM.v = fv_div_by(avg(SR, FL.v) - avg(SL, FR.v) + avg(SLSR, mvR - mvL), den, rden);
+  FM.p = fv_div_by(avg(SR, FL.p) - avg(SL, FR.p) + avg(SLSR, uER - uEL), den, rden);
   const R pM = fv_half(qL.p + qR.p);
   const bool left = fv_ge0(SL);
   const bool right = !left && fv_le0(SR);
@@ -309,6 +328,62 @@ __device__ __forceinline__ void riemann_hllc(const S4<R> &qL, const S4<R> &qR, S
   f.p = mulx<8>(E + sp, su);
 }
 
+// x with its sign changed, a zero as it is: (b - a) from (a - b), whose zero
+// is +0 either way.
+__device__ __forceinline__ double negated_difference(double x) {
+  const uint64_t b = softfp::bits(x);
+  return (b & softfp::MAG) == 0 ? x : softfp::from_bits(b ^ softfp::SIGN);
+}
+
+// The same in binary64, with fewer operations for the same bits:
+//   - max(cL, cR) is the square root of the larger quotient (a correctly
+//     rounded square root is monotone; negative and NaN quotients lose to any
+//     other in both orders);
+//   - S_K - u_K and rho_K (S_K - u_K) of the star state are the negated (left)
+//     or the same (right) difference and product of the wave speeds' step;
+//   - the total energy is formed for the side the flux is taken from only.
+__device__ __forceinline__ void riemann_hllc(const S4<double> &qL, const S4<double> &qR, S4<double> &f, double &pout,
+                                             const Gas<double> &g) {
+  const double rL = qL.r, uL = qL.u, vL = qL.v, pL = qL.p;
+  const double rR = qR.r, uR = qR.u, vR = qR.v, pR = qR.p;
+  const double cmax = softfp::sound_max(pL, rL, pR, rR, g.gamma);
+  const double2 um = softfp::minmax_nm(uL, uR);
+  const double SL = um.x - cmax, SR = um.y + cmax;
+  const double dL = uL - SL, dR = SR - uR;
+  double rcL, rcR, a, b, c, d;
+  mulx2<5>(rL, dL, rR, dR, rcL, rcR);
+  mulx2<1>(rcR, uR, rcL, uL, a, b);
+  mulx2<6>(rcR, pL, rcL, pR, c, d);
+  double uS, pS;
+  fv_div2(a + b + (pL - pR), c + d + mulx<6>(mulx<6>(rcL, rcR), uL - uR), rcR + rcL, uS, pS);
+  const bool sideL = fv_gt0(uS);
+  // branch order of RiemannSolvers.h:89-112
+  const bool bL = fv_gt0(SL);
+  const bool bStar = !bL && (sideL || fv_gt0(SR));
+  const bool left = bL || (bStar && sideL);
+  double sr = left ? rL : rR;
+  double su = left ? uL : uR;
+  const double sv = left ? vL : vR;
+  double sp = left ? pL : pR;
+  const double SK = left ? SL : SR;
+  const double dK = left ? negated_difference(dL) : dR;   // S_K - u_K
+  const double rcK = left ? negated_difference(rcL) : rcR;  // rho_K (S_K - u_K)
+  double E;
+  mulx2<1>(su, su, sv, sv, a, b);
+  mulx2<2>(fv_half(sr), a + b, sp, g.entho, c, d);
+  E = c + d;
+  double rS, ES;
+  mulx2<7>(dK, E, sp, su, a, b);
+  fv_div2(rcK, a - b + mulx<7>(pS, uS), SK - uS, rS, ES);
+  if (bStar) {
+    sr = rS; su = uS; sp = pS; E = ES;
+  }
+  pout = sp;
+  mulx2<1>(sr, su, E + sp, su, f.r, f.p);
+  mulx2<1>(f.r, su, f.r, sv, a, f.v);
+  f.u = a + sp;
+}
+
 // RiemannSolvers.h:130-171 (Kokkos::max / min as (a<b)?b:a and (b<a)?b:a).
 template <class R>
 __device__ __forceinline__ void riemann_fslp(const S4<R> &qL, const S4<R> &qR, S4<R> &f, R &pout, R gdx,
@@ -341,10 +416,11 @@ __device__ __forceinline__ void riemann_fslp(const S4<R> &qL, const S4<R> &qR, S
 
 enum { RS_HLL = 0, RS_HLLC = 1, RS_FSLP = 2 };
 
-template <int RS, class R>
+// VISC: the caller is a viscous kernel (which products run on which pipe)
+template <int RS, bool VISC = false, class R>
 __device__ __forceinline__ void riemann(const S4<R> &qL, const S4<R> &qR, S4<R> &f, R &pout, R gdx, const Gas<R> &g) {
   if constexpr (RS == RS_HLL)
-    riemann_hll(qL, qR, f, pout, g);
+    riemann_hll<VISC>(qL, qR, f, pout, g);
   else if constexpr (RS == RS_FSLP)
     riemann_fslp(qL, qR, f, pout, gdx, g);
   else

@@ -92,7 +92,7 @@ __global__ void ic_kernel(fv2d_params p, int problem, float *U, long long plane,
   init_cell(p, problem, sx, sy, q);
   if (nx) q[1] = -q[1];
   if (ny) q[2] = -q[2];
-  const Gas<double> g{p.gamma0, p.gamma0 - 1.0, 1.0 / (p.gamma0 - 1.0), 0.0};
+  const Gas<double> g = make_gas(p.gamma0, p.gamma0 - 1.0, 1.0 / (p.gamma0 - 1.0), 0.0);
   const S4<double> u = prim_to_cons(S4<double>{q[0], q[1], q[2], q[3]}, g);
   const long long o = (long long)py * pitch + px;
   U[o] = (float)(u.r - (double)bg_r);
@@ -365,7 +365,7 @@ void background(const fv2d_request &r, float *bg_r, float *bg_e) {
   const fv2d_params &p = r.params;
   const int sx = std::max(1, p.Nx / 64), sy = std::max(1, p.Ny / 64);
   std::vector<double> rs, es;
-  const Gas<double> g{p.gamma0, p.gamma0 - 1.0, 1.0 / (p.gamma0 - 1.0), 0.0};
+  const Gas<double> g = make_gas(p.gamma0, p.gamma0 - 1.0, 1.0 / (p.gamma0 - 1.0), 0.0);
   for (int j = sy / 2; j < p.Ny; j += sy)
     for (int i = sx / 2; i < p.Nx; i += sx) {
       double q[4];

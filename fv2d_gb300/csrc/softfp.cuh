@@ -2,250 +2,306 @@
 // correctly rounded division, square root and multiplication, comparisons,
 // fmin / fmax and scalings by powers of two.
 //
-// GB300 executes binary64 at 1/64 of its FP32 rate; a hardware double
-// division or square root occupies that pipe for ~7-8 DFMA-equivalents while
-// the integer pipes stay idle in the FP64 step kernel.  These routines return
-// exactly the IEEE round-to-nearest-even result (the same bits as x / y,
-// sqrt(x), x * y) for finite normal operands with a normal result and for zero
-// operands, and defer every other case (subnormals, infinities, NaNs,
-// division by zero, overflow, underflow) to the hardware instruction.
+// GB300 executes binary64 at 1/64 of its FP32 rate: one warp-wide binary64
+// instruction holds that pipe for as long as ~32-64 integer instructions
+// issue, and a hardware division or square root takes 7-8 of them.  These
+// routines return exactly the IEEE round-to-nearest-even result (the same
+// bits as x / y, sqrt(x), x * y) for finite normal operands with a normal
+// result and for zero operands, and defer every other case (subnormals,
+// infinities, NaNs, division by zero, overflow, underflow) to the hardware
+// instruction.
 //
-// Division: the divisor's 53-bit significand is normalised to a 64-bit word d;
-// its reciprocal word v = floor((2^128 - 1) / d) - 2^64 (the definition of
-// Moller & Granlund, "Improved division by invariant integers", IEEE TC 2011)
-// is seeded from the FP32 reciprocal, refined by two Newton-Raphson steps in
-// 64-bit fixed point and made exact by a final check; their 2-by-1 division
-// step then yields the exact 53-bit quotient and remainder, from which the
-// rounding is decided (compare twice the remainder with the divisor).
+// They are bound by the integer instructions they issue (the ALU pipe takes
+// one warp instruction in two cycles), so each is laid out to need few of
+// them: a 30-bit reciprocal (or reciprocal square root) from the FP32 seed and
+// one Newton step in 32-bit words, the result's 53 bits in two digits of ~30
+// and 23 bits (each digit one 32x32 high product), one exact remainder in
+// 64-bit words that decides the rounding, exponents added in place, and one
+// range test for all operands.  Instructions per call: division 97 (an exact
+// 64-bit reciprocal word, refined and corrected in 128-bit products, took
+// over 200), two quotients by one divisor 151, square root 89, product 59,
+// two products in one call 98.  With them and the shorter HLLC flux of
+// physics.cuh a Kelvin-Helmholtz 2048^2 step (PLM, HLLC) went from 1.66 to
+// 1.10 ms, a Sedov one from 1.33 to 1.01 ms.
 //
-// Division, square root and multiplication are called rather than inlined:
-// the step kernel uses them a dozen times per cell, and one shared copy keeps
-// its code within the instruction caches (measured ~3 % faster).
-//
-// Square root: the FP32 reciprocal square root seeds a Newton-Raphson
-// iteration for 1/sqrt in 64-bit fixed point; the product with the operand
-// gives the integer square root within a few units, which the exact remainder
-// M - S^2 corrects; round up when the remainder exceeds S.
+// The core routines also compile for the host (plain C++), where
+// tests/softfp_harness.cpp runs them against the host's binary64 arithmetic.
 #pragma once
 
 #include <stdint.h>
+#ifndef __CUDACC__
+#include <math.h>
+#include <string.h>
+#endif
+
+#ifdef __CUDACC__
+#define FV2D_SF __host__ __device__ __forceinline__
+#define FV2D_SF_CALL static __host__ __device__ __noinline__
+#else
+#define FV2D_SF inline
+#define FV2D_SF_CALL static
+#endif
 
 namespace fv2d {
 namespace softfp {
 
-// The moves are opaque to the optimiser: a plain bit cast lets it recognise
-// the integer tests below as floating-point classifications and lower them
-// back to binary64 instructions (abs.f64 + setp).
-__device__ __forceinline__ uint64_t bits(double x) {
+#ifndef __CUDACC__
+struct double2 {
+  double x, y;
+};
+inline double2 make_double2(double x, double y) { return double2{x, y}; }
+// units in the last place the host's seeds are moved by (the tests sweep it:
+// the device's approximations are only accurate to an ulp or two)
+static int seed_ulps = 0;
+#endif
+
+// On the device the moves are opaque to the optimiser: a plain bit cast lets
+// it recognise the integer tests below as floating-point classifications and
+// lower them back to binary64 instructions (abs.f64 + setp).
+FV2D_SF uint64_t bits(double x) {
   uint64_t b;
+#ifdef __CUDA_ARCH__
   asm("mov.b64 %0, %1;" : "=l"(b) : "d"(x));
+#else
+  memcpy(&b, &x, 8);
+#endif
   return b;
 }
-__device__ __forceinline__ double from_bits(uint64_t b) {
+FV2D_SF double from_bits(uint64_t b) {
   double x;
+#ifdef __CUDA_ARCH__
   asm("mov.b64 %0, %1;" : "=d"(x) : "l"(b));
+#else
+  memcpy(&x, &b, 8);
+#endif
   return x;
 }
+FV2D_SF uint32_t mulhi32(uint32_t a, uint32_t b) { return (uint32_t)(((uint64_t)a * b) >> 32); }
+
+// FP32 seeds as bit patterns: 1/f and 1/sqrt(f).
+FV2D_SF uint32_t seed_bits(uint32_t fb, bool root) {
+  uint32_t rb;
+#ifdef __CUDA_ARCH__
+  if (root)
+    asm("{\n\t.reg .f32 f, r;\n\tmov.b32 f, %1;\n\trsqrt.approx.ftz.f32 r, f;\n\tmov.b32 %0, r;\n\t}" : "=r"(rb) : "r"(fb));
+  else
+    asm("{\n\t.reg .f32 f, r;\n\tmov.b32 f, %1;\n\trcp.approx.ftz.f32 r, f;\n\tmov.b32 %0, r;\n\t}" : "=r"(rb) : "r"(fb));
+#else
+  float f;
+  memcpy(&f, &fb, 4);
+  const float r = root ? (float)(1.0 / sqrt((double)f)) : (float)(1.0 / (double)f);
+  memcpy(&rb, &r, 4);
+#ifndef __CUDACC__
+  rb += (uint32_t)seed_ulps;
+#endif
+#endif
+  // in [1/2, 1): the 24-bit significand becomes the top of the fixed-point word
+  rb = rb < 0x3F000000u ? 0x3F000000u : rb;
+  return rb > 0x3F7FFFFFu ? 0x3F7FFFFFu : rb;
+}
+
+constexpr uint64_t MAG = 0x7FFFFFFFFFFFFFFFull, INF_BITS = 0x7FF0000000000000ull, SIGN = 0x8000000000000000ull;
+constexpr uint64_t FRAC = 0xFFFFFFFFFFFFFull, ONE52 = 1ull << 52;
 
 // Hardware instructions for the special cases, behind calls so that the
 // compiler cannot if-convert their expansion into the common path (issued
 // predicated-off instructions still occupy the binary64 pipe).
-static __device__ __noinline__ double div_hw(double a, double b) { return a / b; }
-static __device__ __noinline__ double sqrt_hw(double x) { return sqrt(x); }
+FV2D_SF_CALL double div_hw(double a, double b) { return a / b; }
+FV2D_SF_CALL double sqrt_hw(double x) { return sqrt(x); }
+FV2D_SF_CALL double mul_hw(double x, double y) { return x * y; }
+FV2D_SF_CALL bool prod_neg_hw(double x, double y) { return x * y < 0.0; }
 
-// The seeds are assembled from bit fields rather than by int64 <-> float
-// conversions, which issue on the binary64 pipe.
-__device__ __forceinline__ uint64_t recip_word(uint64_t d) {
-  // f = d / 2^63 truncated to 24 bits, in [1, 2); r ~ 1/f in (1/2, 1]
-  const float f = __uint_as_float(0x3F800000u | ((uint32_t)(d >> 40) & 0x7FFFFFu));
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(f));
-  // x = (2 r - 1) 2^64: the fraction field of 2 r shifted up, clamped to
-  // [0, 2^64 - 1] when the approximation leaves [1/2, 1)
-  const uint32_t rb = __float_as_uint(r);
-  uint64_t x = rb >= 0x3F800000u ? ~0ull : rb < 0x3F000000u ? 0ull : (uint64_t)(rb & 0x7FFFFFu) << 41;
-  for (int it = 0; it < 2; ++it) {
-    // e = 2^128 - d (2^64 + x); x += (2^64 + x) e / 2^128
-    const uint64_t lo = d * x, hi = __umul64hi(d, x);
-    const uint64_t s_hi = hi + d;
-    const int64_t e_hi = (int64_t)(0ull - s_hi - (lo != 0));
-    const int64_t corr = e_hi + (int64_t)(__umul64hi(x, (uint64_t)e_hi) - (e_hi < 0 ? x : 0ull));
-    // A Newton step from an overestimate lands below the root by about the
-    // squared error (2^-46 relative after the FP32 seed).  For a divisor
-    // just below a power of two (d > 2^64 - 2^19) the root v is smaller than
-    // that and the step would cross 2^64 + 0, wrapping the fraction word:
-    // clamp at zero, an underestimate the next step refines.
-    x = (corr < 0 && (uint64_t)(-corr) > x) ? 0ull : x + (uint64_t)corr;
-  }
-  // exact: d (2^64 + x) <= 2^128 - 1 < d (2^64 + x + 1)
-#pragma unroll 1
-  for (int k = 0; k < 4; ++k) {
-    const uint64_t lo = d * x, hi = __umul64hi(d, x);
-    const uint64_t s_hi = hi + d;
-    if (s_hi < d) {
-      --x;
-      continue;
-    }
-    const uint64_t lo2 = lo + d;
-    const uint64_t s_hi2 = s_hi + (lo2 < lo);
-    if (s_hi2 < s_hi) break;
-    ++x;
-  }
-  return x;
-}
+FV2D_SF uint32_t hi32(uint64_t x) { return (uint32_t)(x >> 32); }
+FV2D_SF uint32_t lo32(uint64_t x) { return (uint32_t)x; }
+FV2D_SF uint64_t join(uint32_t hi, uint32_t lo) { return ((uint64_t)hi << 32) | lo; }
+constexpr uint32_t EXP_HI = 0x7FF00000u, FRAC_HI = 0xFFFFFu, ONE_HI = 0x100000u, SIGN_HI = 0x80000000u;
 
-// a / b, round to nearest even, in two halves so that quotients with a
-// common divisor share its reciprocal word: div_begin classifies the operands
-// and aligns the dividend, div_finish forms the quotient from v = recip_word(d)
-// (needed only when some quotient takes the fast path).
-struct DivOp {
-  uint64_t ia, ib, d, u1, u0;
-  int e;
-  bool fast;
+FV2D_SF uint64_t significand(uint64_t ib) { return (ib & FRAC) | ONE52; }
+FV2D_SF int exponent(uint64_t ib) { return (int)(hi32(ib) >> 20) & 0x7ff; }
+FV2D_SF bool normal_exp(int e) { return (unsigned)(e - 1) < 0x7FEu; }
+
+// The operand range of the common paths, tested on the high words of all of a
+// routine's operands together (two instructions an operand): biased exponents
+// 768..1279 (adding 256 makes bits 10 and 9 read 10), whose products,
+// quotients, and products divided by a third operand are normal.
+struct Range {
+  uint32_t acc = 0xFFFFFFFFu;
+  FV2D_SF void add(uint64_t x) { acc &= (hi32(x) + 0x10000000u) ^ 0x20000000u; }
+  FV2D_SF bool ok() const { return (acc & 0x60000000u) == 0x60000000u; }
 };
 
-__device__ __forceinline__ DivOp div_begin(double a, double b) {
-  DivOp o;
-  o.ia = bits(a);
-  o.ib = bits(b);
-  const int ea = (int)((o.ia >> 52) & 0x7ff), eb = (int)((o.ib >> 52) & 0x7ff);
-  const uint64_t ma = (o.ia & 0xFFFFFFFFFFFFFull) | (1ull << 52);
-  const uint64_t mb = (o.ib & 0xFFFFFFFFFFFFFull) | (1ull << 52);
+// Reciprocal word of a significand mb in [2^52, 2^53): x = 2^83 / mb with a
+// relative error below 2^-30, x in [2^30, 2^31].  With B = mb / 2^21
+// truncated to 32 bits, X0 = 2^32 (1 + e) 2^31 / B from the seed (|e| < 2^-21:
+// 24-bit truncation of B and two ulps of the approximation), one Newton step
+// X0 (2 - B X0 / 2^63) / 2 leaves e^2 < 2^-42 and three truncations of
+// 2^-31 each.
+FV2D_SF uint32_t recip_word(uint64_t mb) {
+  const uint32_t B = (uint32_t)(mb >> 21);
+  const uint32_t X0 = (seed_bits(0x3F800000u | ((B >> 8) & 0x7FFFFFu), false) << 8) | 0x80000000u;
+  return mulhi32(X0, 0u - mulhi32(B, X0));
+}
+
+// n / mb rounded to nearest, as a 53-bit integer Q = n 2^52 / mb, for n in
+// [mb, 2 mb) (n below 2^54) and x = recip_word(mb).  The high digit qa (30
+// bits, scale 2^-29) is taken one below its estimate: the estimate is off by
+// (-3, 1) units, so the remainder r1 = (n 2^29 - qa mb) lies in (0, 4 mb),
+// below 2^55.  The low digit qb (scale 2^-52) is rounded to nearest with an
+// error of 0.58, so |r2| < 0.58 mb and one step either way rounds Q.  A
+// quotient of two 53-bit significands is never midway between two results
+// ((2 Q + 1) mb = 2^53 n would need 2^53 | mb), so there are no ties.
+FV2D_SF uint64_t quotient(uint64_t n, uint64_t mb, uint32_t x) {
+  const uint32_t qa = mulhi32((uint32_t)(n >> 22), x) - 1u;
+  const uint64_t r1 = (n << 29) - (uint64_t)qa * mb;
+  const uint32_t qb = (mulhi32((uint32_t)(r1 >> 23), x) + 16u) >> 5;
+  const int64_t r2 = (int64_t)((r1 << 23) - (uint64_t)qb * mb) * 2;
+  uint64_t Q = ((uint64_t)qa << 23) + qb;
+  Q += r2 > (int64_t)mb ? 1u : 0u;
+  Q -= r2 < -(int64_t)mb ? 1u : 0u;
+  return Q;
+}
+
+// The sign of s's bit 31 on a positive high word.
+FV2D_SF uint32_t with_sign(uint32_t h, uint32_t s) { return h | (s & SIGN_HI); }
+
+// a / b for normal a, b with a normal quotient, x = recip_word of b's
+// significand.  Exponents stay in place in the high words; a significand of
+// 2^53 carries into the exponent.
+FV2D_SF double div_core(uint64_t a, uint64_t b, uint32_t x) {
+  const uint64_t ma = significand(a), mb = significand(b);
   const bool big = ma >= mb;
-  o.e = ea - eb + 1023 - (big ? 0 : 1);
-  o.fast = !(ea == 0 || ea == 0x7ff || eb == 0 || eb == 0x7ff || o.e <= 0 || o.e >= 0x7fe);
-  // Q = floor(n 2^52 / mb) with n = ma or 2 ma, i.e. (n 2^63) / (mb 2^11)
-  o.d = mb << 11;
-  const uint64_t n = big ? ma : (ma << 1);
-  o.u1 = n >> 1;
-  o.u0 = n << 63;
-  return o;
+  const uint64_t Q = quotient(big ? ma : ma << 1, mb, x);
+  const uint32_t h = hi32(Q) + (hi32(a) & EXP_HI) - (hi32(b) & EXP_HI) + (big ? 1022u << 20 : 1021u << 20);
+  return from_bits(join(with_sign(h, hi32(a) ^ hi32(b)), lo32(Q)));
 }
+// Operands outside the common range: zeros (quiescent regions: a zero with
+// the xor of the signs), else the hardware instruction.
+FV2D_SF double div_rare(double a, double b) {
+  const uint64_t ia = bits(a), ib = bits(b);
+  if ((ia & MAG) == 0 && normal_exp(exponent(ib))) return from_bits((ia ^ ib) & SIGN);
+  return div_hw(a, b);
+}
+FV2D_SF double div_with(double a, double b, uint32_t x) {
+  Range r;
+  r.add(bits(a));
+  r.add(bits(b));
+  if (!r.ok()) return div_rare(a, b);
+  return div_core(bits(a), bits(b), x);
+}
+// the reciprocal word of b, for any b (meaningless unless b is normal)
+FV2D_SF uint32_t recip_of(double b) { return recip_word(significand(bits(b))); }
 
-__device__ __forceinline__ double div_finish(const DivOp &o, double a, double b, uint64_t v) {
-  if (!o.fast) {
-    // +-0 / (finite nonzero normal) is a zero with the xor of the signs;
-    // quiescent regions (zero momentum) make this the common special case.
-    const int eb = (int)((o.ib >> 52) & 0x7ff);
-    if ((o.ia << 1) == 0 && eb != 0 && eb != 0x7ff) return from_bits((o.ia ^ o.ib) & 0x8000000000000000ull);
-    return div_hw(a, b);
-  }
-  const uint64_t d = o.d, u1 = o.u1, u0 = o.u0;
-  uint64_t q0 = v * u1, q1 = __umul64hi(v, u1);
-  const uint64_t s0 = q0 + u0;
-  q1 = q1 + u1 + (s0 < q0) + 1;
-  q0 = s0;
-  uint64_t r = u0 - q1 * d;
-  if (r > q0) {
-    --q1;
-    r += d;
-  }
-  if (r >= d) {
-    ++q1;
-    r -= d;
-  }
-  // nearest even: compare 2 r with d
-  uint64_t Q = q1 + ((r > d - r) || (r == d - r && (q1 & 1)));
-  int e = o.e;
-  if (Q >> 53) {
-    Q >>= 1;
-    ++e;
-  }
-  const uint64_t out = ((uint64_t)e << 52) | (Q & 0xFFFFFFFFFFFFFull) | ((o.ia ^ o.ib) & 0x8000000000000000ull);
-  return from_bits(out);
-}
-
-static __device__ __noinline__ double div_rn(double a, double b) {
-  const DivOp o = div_begin(a, b);
-  const uint64_t v = o.fast ? recip_word(o.d) : 0ull;
-  return div_finish(o, a, b, v);
-}
+// Division, square root and multiplication are called rather than inlined:
+// the step kernel uses them dozens of times per cell, and one shared copy
+// keeps its code within the instruction caches.
+FV2D_SF_CALL double div_rn(double a, double b) { return div_with(a, b, recip_of(b)); }
 
 // {a1 / b, a2 / b} (returned by value: outputs through references would live
 // on the stack across the call)
-static __device__ __noinline__ double2 div2_rn(double a1, double a2, double b) {
-  const DivOp o1 = div_begin(a1, b), o2 = div_begin(a2, b);
-  const uint64_t v = (o1.fast || o2.fast) ? recip_word(o1.d) : 0ull;
-  return make_double2(div_finish(o1, a1, b, v), div_finish(o2, a2, b, v));
+FV2D_SF_CALL double2 div2_rn(double a1, double a2, double b) {
+  const uint32_t x = recip_of(b);
+  Range r;
+  r.add(bits(a1));
+  r.add(bits(a2));
+  r.add(bits(b));
+  if (!r.ok()) return make_double2(div_with(a1, b, x), div_with(a2, b, x));
+  return make_double2(div_core(bits(a1), bits(b), x), div_core(bits(a2), bits(b), x));
 }
 
-// Quotients by one divisor b: recip_of(b) computes its reciprocal word once
-// (0 when b is zero, subnormal, infinite or NaN: the hardware handles every
-// quotient by such a b), div_by(a, b, v) forms each quotient.
-static __device__ __noinline__ uint64_t recip_of(double b) {
-  const uint64_t ib = bits(b);
-  const int eb = (int)((ib >> 52) & 0x7ff);
-  if (eb == 0 || eb == 0x7ff) return 0ull;
-  return recip_word(((ib & 0xFFFFFFFFFFFFFull) | (1ull << 52)) << 11);
-}
-static __device__ __noinline__ double div_by(double a, double b, uint64_t v) {
-  const DivOp o = div_begin(a, b);
-  // a normal divisor's reciprocal word is never 0 (it is at least 2^11)
-  if (o.fast && v == 0ull) return div_rn(a, b);
-  return div_finish(o, a, b, v);
-}
+// Quotients by one divisor b: recip_of(b) forms its reciprocal word once,
+// div_by(a, b, x) each quotient.
+FV2D_SF_CALL double div_by(double a, double b, uint32_t x) { return div_with(a, b, x); }
 
-// recip_of(b) for a divisor known on the host (the mesh spacings): the same
-// word from its definition, floor((2^128 - 1) / d) - 2^64 with d the
-// divisor's significand aligned to bit 63; the quotient lies in
-// [2^64, 2^65), so its low 64 bits are the word.
-inline uint64_t recip_of_host(double b) {
+// recip_of(b) for a divisor known on the host (the mesh spacings): 2^83 / mb
+// rounded down.
+inline uint32_t recip_of_host(double b) {
   union {
     double f;
     uint64_t u;
   } c{b};
-  const int eb = (int)((c.u >> 52) & 0x7ff);
-  if (eb == 0 || eb == 0x7ff) return 0ull;
-  const uint64_t d = ((c.u & 0xFFFFFFFFFFFFFull) | (1ull << 52)) << 11;
-  return (uint64_t)(~(unsigned __int128)0 / d);
+  return (uint32_t)(((unsigned __int128)1 << 83) / ((c.u & FRAC) | ONE52));
 }
 
-// sqrt(x), round to nearest even.
-static __device__ __noinline__ double sqrt_rn(double x) {
+// sqrt of the significand: M = m 2^(52 + odd) in [2^104, 2^106), g = M 2^-104;
+// S = sqrt(M) rounded to nearest, in [2^52, 2^53].  Y = 2^31 / sqrt(g) to
+// 2^-29.4 (one Newton step from the seed), the high digit S1 (scale 2^-29)
+// two below its estimate, which is off by (-3, 1.5), so r1 = M 2^-46 - S1^2 is
+// positive and below 2^34; the low digit's error is below 0.85 (rounding 0.5,
+// second-order term 0.2, truncations), and the exact remainder R = M - S^2
+// (its low 64 bits carry it) settles the rounding: a step up when R > S, down
+// when R <= -S.
+FV2D_SF uint64_t root(uint64_t m, int odd) {
+  const uint32_t Z = (uint32_t)(m >> (22 - odd));  // g 2^30
+  const uint32_t g = ((uint32_t)(127 + odd) << 23) | ((uint32_t)(m >> 29) & 0x7FFFFFu);
+  const uint32_t X0 = (seed_bits(g, true) << 8) | 0x80000000u;
+  const uint32_t U = mulhi32(mulhi32(X0, X0), Z);
+  const uint32_t Y = mulhi32(X0, 0xC0000000u - U);
+  const uint32_t S1 = mulhi32(Z, Y) - 2u;
+  const uint64_t r1 = (m << (6 + odd)) - (uint64_t)S1 * S1;
+  const uint32_t S2 = (mulhi32((uint32_t)(r1 >> 2), Y) + 8u) >> 4;
+  const uint64_t S = ((uint64_t)S1 << 23) + S2;
+  const int64_t R = (int64_t)(join((uint32_t)m << (20 + odd), 0u) - S * S);
+  return S + (R > (int64_t)S ? 1u : 0u) - (R <= -(int64_t)S ? 1u : 0u);
+}
+
+// sqrt(x) of a positive normal x, round to nearest even.
+FV2D_SF double sqrt_core(uint64_t ix) {
+  const int E = (int)(hi32(ix) >> 20);
+  const int odd = (E & 1) ^ 1;  // x = m 2^(E - 1075), E - 1075 - odd even
+  const uint64_t S = root(significand(ix), odd);
+  return from_bits(S + join((uint32_t)((E - odd + 1021) >> 1) << 20, 0u));
+}
+FV2D_SF_CALL double sqrt_rn(double x) {
   const uint64_t ix = bits(x);
-  const int E = (int)(ix >> 52);  // sign bit included: negative values fail the range test
-  if ((ix << 1) == 0) return x;   // sqrt(+-0) = +-0
-  if (E == 0 || E >= 0x7ff) return sqrt_hw(x);
-  const uint64_t m = (ix & 0xFFFFFFFFFFFFFull) | (1ull << 52);
-  const int t = E - 1075;  // x = m 2^t
-  const int odd = t & 1;
-  // M = m 2^(52 + odd) in [2^104, 2^106); S = floor(sqrt(M)) in [2^52, 2^53)
-  const uint64_t Z = m << (10 + odd);  // M / 2^42, in [2^62, 2^64)
-  // Y ~ 2^94 / sqrt(Z), in (2^62, 2^63]: with g = Z / 2^62 = (m / 2^52) 2^odd
-  // in [1, 4) truncated to 24 bits, Y = rsqrt(g) 2^63 and rsqrt(g) in (1/2, 1]
-  const float g = __uint_as_float((uint32_t)((127 + odd) << 23) | (uint32_t)((m >> 29) & 0x7FFFFFu));
-  float rs;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rs) : "f"(g));
-  const uint32_t sb = __float_as_uint(rs);
-  uint64_t Y = (uint64_t)((sb & 0x7FFFFFu) | 0x800000u) << (39 + (int)(sb >> 23) - 126);
-  for (int it = 0; it < 2; ++it) {
-    // U = Z Y^2 / 2^128 ~ 2^60; Y <- Y (3 2^60 - U) / 2^61
-    const uint64_t W = __umul64hi(Y, Y);
-    const uint64_t U = __umul64hi(Z, W);
-    Y = __umul64hi(Y, (0x3000000000000000ull - U) << 2) << 1;
-  }
-  // sqrt(M) = sqrt(Z) 2^21 = Z Y / 2^73
-  uint64_t S = __umul64hi(Z, Y) >> 9;
-  // exact remainder R = M - S^2 (small; the low 64 bits carry it)
-  const uint64_t Mlo = m << (52 + odd);
-  int64_t R = (int64_t)(Mlo - S * S);
-#pragma unroll 1
-  for (int k = 0; k < 4 && R < 0; ++k) {
-    R += (int64_t)(2 * S - 1);
-    --S;
-  }
-#pragma unroll 1
-  for (int k = 0; k < 4 && R > (int64_t)(2 * S); ++k) {
-    R -= (int64_t)(2 * S + 1);
-    ++S;
-  }
-  uint64_t Q = S + (R > (int64_t)S);
-  int e = ((t - odd) >> 1) + 26 + 1023;  // sqrt(x) = Q 2^((t - odd)/2 - 26), Q in [2^52, 2^53]
-  if (Q >> 53) {
-    Q >>= 1;
-    ++e;
-  }
-  return from_bits(((uint64_t)e << 52) | (Q & 0xFFFFFFFFFFFFFull));
+  if ((ix << 1) == 0) return x;  // sqrt(+-0) = +-0
+  if (!normal_exp((int)(ix >> 52))) return sqrt_hw(x);  // sign bit included: negative values fail the test
+  return sqrt_core(ix);
+}
+
+// x * y, round to nearest even, for normal operands with a normal result:
+// the 106-bit product of the significands, one of them aligned to bit 63 so
+// that the product's high 64 bits hold the result's 52 or 53 bits and the low
+// ones decide the rounding.
+FV2D_SF double mul_core(uint64_t a, uint64_t b) {
+  const uint64_t A = (a << 11) | SIGN;
+  const uint32_t al = lo32(A), ah = hi32(A), bl = lo32(b), bh = (hi32(b) & FRAC_HI) | ONE_HI;
+  const uint64_t p0 = (uint64_t)al * bl;
+  const uint64_t p1 = (uint64_t)ah * bl + hi32(p0);
+  const uint64_t p2 = (uint64_t)al * bh + lo32(p1);
+  const uint64_t H = (uint64_t)ah * bh + hi32(p1) + hi32(p2);  // in [2^51, 2^53)
+  const uint32_t top = hi32(H) & ONE_HI;                       // product of the significands >= 2
+  const int k = top ? 0 : 1;
+  const uint32_t F = (uint32_t)(((join(lo32(p2), lo32(p0))) << k) >> 32), G = lo32(p0) << k;
+  uint64_t M = join((uint32_t)((H << k) >> 32), (uint32_t)((join(lo32(H), lo32(p2)) << k) >> 32)) + (F >> 31);
+  if (((F ^ 0x80000000u) | G) == 0) M &= ~1ull;  // tie: to even
+  const uint32_t h = hi32(M) + (hi32(a) & EXP_HI) + (hi32(b) & EXP_HI) + top - (1024u << 20);
+  return from_bits(join(with_sign(h, hi32(a) ^ hi32(b)), lo32(M)));
+}
+// Operands outside the common range: zero times finite (zero velocities)
+// keeps the xor of the signs, the rest takes the hardware instruction.
+FV2D_SF double mul_rare(double x, double y) {
+  const uint64_t a = bits(x), b = bits(y);
+  if (((a & MAG) == 0 || (b & MAG) == 0) && exponent(a) != 0x7FF && exponent(b) != 0x7FF)
+    return from_bits((a ^ b) & SIGN);
+  return mul_hw(x, y);
+}
+FV2D_SF double mul_with(double x, double y) {
+  Range r;
+  r.add(bits(x));
+  r.add(bits(y));
+  if (!r.ok()) return mul_rare(x, y);
+  return mul_core(bits(x), bits(y));
+}
+FV2D_SF_CALL double mul_rn(double x, double y) { return mul_with(x, y); }
+// two independent products in one call
+FV2D_SF_CALL double2 mul2_rn(double x0, double y0, double x1, double y1) {
+  Range r;
+  r.add(bits(x0));
+  r.add(bits(y0));
+  r.add(bits(x1));
+  r.add(bits(y1));
+  if (!r.ok()) return make_double2(mul_with(x0, y0), mul_with(x1, y1));
+  return make_double2(mul_core(bits(x0), bits(y0)), mul_core(bits(x1), bits(y1)));
 }
 
 // ---------------------------------------------------------------------------
@@ -256,115 +312,105 @@ static __device__ __noinline__ double sqrt_rn(double x) {
 // subnormal, overflow, NaN/inf inputs of a product) go to the hardware
 // instruction through a call that is not if-converted.
 
-
-
-constexpr uint64_t MAG = 0x7FFFFFFFFFFFFFFFull, INF_BITS = 0x7FF0000000000000ull, SIGN = 0x8000000000000000ull;
-
-__device__ __forceinline__ bool isnan_b(uint64_t b) { return (b & MAG) > INF_BITS; }
-
-static __device__ __noinline__ double mul_hw(double x, double y) { return x * y; }
-static __device__ __noinline__ bool prod_neg_hw(double x, double y) { return x * y < 0.0; }
+FV2D_SF bool isnan_b(uint64_t b) { return (b & MAG) > INF_BITS; }
 
 // x > 0, x < 0, x >= 0, x <= 0
-__device__ __forceinline__ bool gt0(double x) { return bits(x) - 1ull < INF_BITS; }
-__device__ __forceinline__ bool lt0(double x) { return bits(x) - (SIGN + 1ull) < INF_BITS; }
-__device__ __forceinline__ bool ge0(double x) {
+FV2D_SF bool gt0(double x) { return bits(x) - 1ull < INF_BITS; }
+FV2D_SF bool lt0(double x) { return bits(x) - (SIGN + 1ull) < INF_BITS; }
+FV2D_SF bool ge0(double x) {
   const uint64_t b = bits(x);
   return b <= INF_BITS || b == SIGN;
 }
-__device__ __forceinline__ bool le0(double x) {
+FV2D_SF bool le0(double x) {
   const uint64_t b = bits(x);
   return (b & MAG) == 0 || b - SIGN <= INF_BITS;
 }
 
 // Order key with -0 == +0 (IEEE comparison order for non-NaN values).
-__device__ __forceinline__ int64_t key_ieee(uint64_t b) {
+FV2D_SF int64_t key_ieee(uint64_t b) {
   const int64_t m = (int64_t)(b & MAG);
   return (int64_t)b < 0 ? -m : m;
 }
 // x < y (IEEE: false when either is NaN)
-__device__ __forceinline__ bool lt(double x, double y) {
+FV2D_SF bool lt(double x, double y) {
   const uint64_t a = bits(x), b = bits(y);
   return !isnan_b(a) && !isnan_b(b) && key_ieee(a) < key_ieee(b);
 }
 
 // maximumNumber / minimumNumber: a NaN operand yields the other one; -0 < +0.
 // (The C fmax / fmin of the aarch64 C library, FMAXNM / FMINNM.)
-__device__ __forceinline__ int64_t key_total(uint64_t b) { return (int64_t)(b ^ ((uint64_t)((int64_t)b >> 63) >> 1)); }
-__device__ __forceinline__ double fmax_nm(double x, double y) {
+FV2D_SF int64_t key_total(uint64_t b) { return (int64_t)(b ^ ((uint64_t)((int64_t)b >> 63) >> 1)); }
+FV2D_SF double fmax_nm(double x, double y) {
   const uint64_t a = bits(x), b = bits(y);
   if (isnan_b(b)) return x;
   if (isnan_b(a)) return y;
   return key_total(a) > key_total(b) ? x : y;
 }
-__device__ __forceinline__ double fmin_nm(double x, double y) {
+FV2D_SF double fmin_nm(double x, double y) {
   const uint64_t a = bits(x), b = bits(y);
   if (isnan_b(b)) return x;
   if (isnan_b(a)) return y;
   return key_total(a) < key_total(b) ? x : y;
 }
+// {fmin_nm(x, y), fmax_nm(x, y)} from one comparison
+FV2D_SF double2 minmax_nm(double x, double y) {
+  const uint64_t a = bits(x), b = bits(y);
+  if (isnan_b(b)) return make_double2(x, x);
+  if (isnan_b(a)) return make_double2(y, y);
+  const bool less = key_total(a) < key_total(b);
+  return make_double2(less ? x : y, less ? y : x);
+}
 
 // |x| < |y|
-__device__ __forceinline__ bool lt_abs(double x, double y) {
+FV2D_SF bool lt_abs(double x, double y) {
   const uint64_t a = bits(x) & MAG, b = bits(y) & MAG;
   return a < b && b <= INF_BITS;
 }
 
 // x * y < 0.  Nonzero non-NaN factors of opposite signs give a negative
 // product unless it underflows to -0, impossible when the biased exponents
-// sum to at least 972 (|x y| >= 2^-1074); smaller products go to hardware.
-__device__ __forceinline__ bool prod_neg(double x, double y) {
-  const uint64_t a = bits(x), b = bits(y);
-  const uint64_t ma = a & MAG, mb = b & MAG;
-  if (!((a ^ b) & SIGN) || ma == 0 || mb == 0 || ma > INF_BITS || mb > INF_BITS) return false;
-  const int ea = (int)(ma >> 52), eb = (int)(mb >> 52);
-  if (ea != 0 && eb != 0 && ea + eb >= 972) return true;
+// sum to at least 972 (|x y| >= 2^-1074); smaller products, zeros, subnormals,
+// infinities and NaNs go through the call.
+FV2D_SF bool prod_neg(double x, double y) {
+  const uint32_t a = (uint32_t)(bits(x) >> 32), b = (uint32_t)(bits(y) >> 32);
+  if (!((a ^ b) >> 31)) return false;
+  const uint32_t xa = a & 0x7FF00000u, xb = b & 0x7FF00000u;
+  if (xa - 1u < 0x7FEFFFFFu && xb - 1u < 0x7FEFFFFFu && xa + xb >= (972u << 20)) return true;
+  if ((bits(x) & MAG) == 0 || (bits(y) & MAG) == 0) return false;
   return prod_neg_hw(x, y);
 }
 
 // x * 2^k for y == 2^k (k = unbiased exponent of y): exact exponent shift
 // when x and the result are normal; zeros keep their sign.
-__device__ __forceinline__ double mul_pow2(double x, double y, int k) {
+FV2D_SF double mul_pow2(double x, double y, int k) {
   const uint64_t a = bits(x);
-  const int e = (int)((a >> 52) & 0x7FF);
+  const int e = exponent(a);
+  if (normal_exp(e) && normal_exp(e + k)) return from_bits(a + ((uint64_t)((uint32_t)k << 20) << 32));
   if ((a & MAG) == 0) return x;
-  if ((unsigned)(e - 1) < 0x7FEu && (unsigned)(e + k - 1) < 0x7FEu) return from_bits(a + ((uint64_t)(int64_t)k << 52));
   return mul_hw(x, y);
 }
 
 // x * 0.5
-__device__ __forceinline__ double half(double x) { return mul_pow2(x, 0.5, -1); }
+FV2D_SF double half(double x) { return mul_pow2(x, 0.5, -1); }
 
-// x * y, round to nearest even, for normal operands with a normal result
-// (and zero times finite): the 106-bit product of the significands, cut at
-// bit 52 or 53 with the remainder deciding the rounding.  Subnormal, infinite
-// or NaN operands and results that overflow or fall below 2^-1022 (where the
-// subnormal grid changes the rounding) use the hardware instruction.
-static __device__ __noinline__ double mul_rn(double x, double y) {
-  const uint64_t a = bits(x), b = bits(y);
-  const uint64_t sgn = (a ^ b) & SIGN;
-  const int ea = (int)((a >> 52) & 0x7FF), eb = (int)((b >> 52) & 0x7FF);
-  if ((a & MAG) == 0 || (b & MAG) == 0) {
-    if (ea != 0x7FF && eb != 0x7FF) return from_bits(sgn);
-    return mul_hw(x, y);
-  }
-  int e = ea + eb - 1023;
-  if ((unsigned)(ea - 1) >= 0x7FEu || (unsigned)(eb - 1) >= 0x7FEu || (unsigned)(e - 1) >= 0x7FDu)
-    return mul_hw(x, y);
-  const uint64_t ma = (a & 0xFFFFFFFFFFFFFull) | (1ull << 52), mb = (b & 0xFFFFFFFFFFFFFull) | (1ull << 52);
-  const uint64_t lo = ma * mb, hi = __umul64hi(ma, mb);  // P = hi 2^64 + lo in [2^104, 2^106)
-  const int top = (int)(hi >> 41);                        // bit 105 of P
-  e += top;
-  const int s = 52 + top;
-  uint64_t M = (hi << (64 - s)) | (lo >> s);              // P >> s in [2^52, 2^53)
-  const uint64_t R = lo & ((1ull << s) - 1), H = 1ull << (s - 1);
-  M += (R > H) || (R == H && (M & 1));
-  if (M >> 53) {
-    M >>= 1;
-    ++e;
-  }
-  if (e >= 0x7FF) return mul_hw(x, y);
-  return from_bits(sgn | ((uint64_t)e << 52) | (M & 0xFFFFFFFFFFFFFull));
+// sqrt(fmax_nm(gamma pL / rL, gamma pR / rR)), each operation rounded: the
+// larger sound speed of two states, in one call with two independent chains.
+// Positive operands of that range keep every intermediate normal.
+FV2D_SF_CALL double sound_max_rare(double pL, double rL, double pR, double rR, double gamma) {
+  return sqrt_rn(fmax_nm(div_rn(mul_rn(pL, gamma), rL), div_rn(mul_rn(pR, gamma), rR)));
+}
+FV2D_SF_CALL double sound_max(double pL, double rL, double pR, double rR, double gamma) {
+  Range r;
+  r.add(bits(pL));
+  r.add(bits(rL));
+  r.add(bits(pR));
+  r.add(bits(rR));
+  r.add(bits(gamma));
+  const uint32_t signs = hi32(bits(pL)) | hi32(bits(rL)) | hi32(bits(pR)) | hi32(bits(rR)) | hi32(bits(gamma));
+  if (!r.ok() || (int32_t)signs < 0) return sound_max_rare(pL, rL, pR, rR, gamma);
+  const uint64_t a = bits(div_core(bits(mul_core(bits(gamma), bits(pL))), bits(rL), recip_of(rL)));
+  const uint64_t b = bits(div_core(bits(mul_core(bits(gamma), bits(pR))), bits(rR), recip_of(rR)));
+  return sqrt_core(a > b ? a : b);
 }
 
 }  // namespace softfp

@@ -77,7 +77,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, int *err_flag, 
   return false;
 }
 
-__device__ __forceinline__ double ddivc(double x, double d, double inv_d, int pow2, uint64_t rw) {
+__device__ __forceinline__ double ddivc(double x, double d, double inv_d, int pow2, uint32_t rw) {
   // x / d; when 1/d is exactly representable the product is the same
   // correctly rounded value; otherwise the quotient uses d's reciprocal word
   // rw, formed once on the host.
@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(NT, step_ctas_per_sm<RECON, RS>(VISC))
       }
       S4<double> fl;
       double pout;
-      riemann<RS>(qL, qR, fl, pout, ydir ? a.gy_dy : a.gx_dx, gas);
+      riemann<RS, VISC>(qL, qR, fl, pout, ydir ? a.gy_dy : a.gx_dx, gas);
       if (!ydir) {
         const int F = L::FX + r * (TX + 1) + c;
         SMI(F) = fl.r;
