@@ -27,7 +27,7 @@
 
 namespace fv2d {
 cudaError_t init_step_kernels();
-cudaError_t launch_step(int rs, int recon, dim3 grid, cudaStream_t s, const CUtensorMap &t0, const CUtensorMap &t1,
+cudaError_t launch_step(int tile, int rs, int recon, dim3 grid, cudaStream_t s, const CUtensorMap &t0, const CUtensorMap &t1,
                         const StepArgs &a);
 cudaError_t launch_commit(cudaStream_t s, const StepArgs &a);
 }
@@ -38,6 +38,7 @@ struct fv2d_ctx {
   fv2d_params p;
   int device = 0;
   cudaStream_t own_stream = nullptr, stream = nullptr;
+  int tile = TILE_WIDE;  // TILE_* of the step (choose_tile)
   int pitch = 0;
   long long plane = 0;
   double *Q[2] = {nullptr, nullptr};
@@ -259,6 +260,23 @@ int sync_state(fv2d_ctx *ctx) {
 // been queued since (a set_prim followed by compute_dt needs one round trip).
 int fresh_state(fv2d_ctx *ctx) { return ctx->st_fresh ? FV2D_OK : sync_state(ctx); }
 
+template <class T>
+dim3 grid_of(const fv2d_params &p) {
+  return dim3((p.Nx + T::TX - 1) / T::TX, (p.Ny + T::TY - 1) / T::TY);
+}
+// The tile of a grid.  A small tile's CTA is done in half a wide one's time
+// but does a quarter of its cells, so it pays while all of them fit the chip
+// at about three to an SM (us a step, wide | small: Sod 512 x 8, 64 small
+// tiles, 27 | 18; KH 64^2, 64, 33 | 25; 128^2, 256, 33 | 27; 192^2, 576,
+// 35 | 34; 256^2, 1024, 40 | 52).
+int choose_tile(const fv2d_params &p) {
+  const dim3 g = grid_of<SmallTile>(p);
+  return (long long)g.x * g.y <= 3 * 152 ? TILE_SMALL : TILE_WIDE;
+}
+dim3 tile_grid(const fv2d_ctx *c) {
+  return c->tile == TILE_SMALL ? grid_of<SmallTile>(c->p) : grid_of<WideTile>(c->p);
+}
+
 void fill_args(fv2d_ctx *c) {
   const fv2d_params &p = c->p;
   StepArgs &a = c->args;
@@ -275,8 +293,8 @@ void fill_args(fv2d_ctx *c) {
   a.pitch = c->pitch;
   a.Nx = p.Nx;
   a.Ny = p.Ny;
-  const int gx = (p.Nx + TX - 1) / TX, gy = (p.Ny + TY - 1) / TY;
-  a.nblocks = gx * gy;
+  const dim3 grid = tile_grid(c);
+  a.nblocks = grid.x * grid.y;
   a.gamma = p.gamma0;
   a.gm1 = p.gamma0 - 1.0;
   a.entho = 1.0 / (p.gamma0 - 1.0);
@@ -324,16 +342,16 @@ int launch_update(fv2d_ctx *ctx, int driven, double dt) {
   a.driven = driven;
   a.dt_arg = dt;
   a.mirror = driven ? nullptr : ctx->mirror_dev;  // captured device loops never write it
-  const dim3 grid((ctx->p.Nx + TX - 1) / TX, (ctx->p.Ny + TY - 1) / TY);
+  const dim3 grid = tile_grid(ctx);
   const int rk = recon_kind(ctx->p.reconstruction);
   if (ctx->p.time_stepping == FV2D_TS_EULER) {
     a.stage = STAGE_EULER;
-    CK(launch_step(ctx->p.riemann_solver, rk, grid, ctx->stream, ctx->tm[0], ctx->tm[1], a));
+    CK(launch_step(ctx->tile, ctx->p.riemann_solver, rk, grid, ctx->stream, ctx->tm[0], ctx->tm[1], a));
   } else {
     a.stage = STAGE_RK2_PREDICT;
-    CK(launch_step(ctx->p.riemann_solver, rk, grid, ctx->stream, ctx->tm[0], ctx->tm[1], a));
+    CK(launch_step(ctx->tile, ctx->p.riemann_solver, rk, grid, ctx->stream, ctx->tm[0], ctx->tm[1], a));
     a.stage = STAGE_RK2_CORRECT;
-    CK(launch_step(ctx->p.riemann_solver, rk, grid, ctx->stream, ctx->tm[0], ctx->tm[1], a));
+    CK(launch_step(ctx->tile, ctx->p.riemann_solver, rk, grid, ctx->stream, ctx->tm[0], ctx->tm[1], a));
   }
   CK(launch_commit(ctx->stream, a));
   return FV2D_OK;
@@ -397,7 +415,9 @@ int encode_maps(fv2d_ctx *ctx) {
   for (int b = 0; b < 2; ++b) {
     cuuint64_t dims[3] = {(cuuint64_t)(p.Nx + 4), (cuuint64_t)(p.Ny + 4), 4};
     cuuint64_t strides[2] = {(cuuint64_t)ctx->pitch * sizeof(double), (cuuint64_t)ctx->plane * sizeof(double)};
-    cuuint32_t box[3] = {(cuuint32_t)SW, (cuuint32_t)SH, 4};
+    const bool small = ctx->tile == TILE_SMALL;
+    cuuint32_t box[3] = {(cuuint32_t)(small ? SmallTile::SW : WideTile::SW),
+                         (cuuint32_t)(small ? SmallTile::SH : WideTile::SH), 4};
     cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = enc(&ctx->tm[b], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, ctx->Q[b], dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -464,7 +484,7 @@ const char *fv2d_last_error(fv2d_ctx *ctx) {
 int fv2d_build_info(char *buf, int len) {
   if (!buf || len <= 0) return FV2D_ERR_INVALID;
   std::snprintf(buf, (size_t)len, "fv2d_gpu fp64 step: tile %dx%d, %d threads/CTA, halo %d, sm_103a, TMA 3-D box %dx%dx4",
-                TX, TY, NT, HALO, SW, SH);
+                WideTile::TX, WideTile::TY, WideTile::NT, HALO, WideTile::SW, WideTile::SH);
   return FV2D_OK;
 }
 
@@ -501,6 +521,7 @@ int fv2d_create(const fv2d_params *p, int device, fv2d_ctx **out) {
     return bail(cuda_fail(ctx, e, "cudaStreamCreate"));
   ctx->stream = ctx->own_stream;
 
+  ctx->tile = choose_tile(*p);
   const int W = p->Nx + 4, H = p->Ny + 4;
   ctx->pitch = (W + 31) / 32 * 32;
   ctx->plane = (long long)H * ctx->pitch;

@@ -117,7 +117,7 @@ __host__ __device__ __forceinline__ bool fv_isnan(float x) { return isnan(x); }
 // Products moved from the binary64 pipe to the integer pipes (softfp::mul_rn),
 // by group: a product holds the binary64 pipe for 64 cycles of an SM
 // sub-partition, an integer-pipe one the ALU for about as long, so the set
-// that balances the two is the fastest.  FV2D_SOFT_MUL is a mask (bit
+// that balances the two is the fastest.  The set is a mask (bit
 // GROUP - 1 set: that group on the integer pipes); the groups are
 //   1  HLLC: squared velocities, p gamma, u* numerator, fluxes
 //   2  HLLC: total energy (rho/2 (u^2 + v^2), p / (gamma - 1))
@@ -141,23 +141,56 @@ __host__ __device__ __forceinline__ bool fv_isnan(float x) { return isnan(x); }
 #ifndef FV2D_SOFT_MUL
 #define FV2D_SOFT_MUL 14607
 #endif
-template <int GROUP, class R>
+constexpr int kSoftMul = FV2D_SOFT_MUL, kSoftMulVisc = FV2D_SOFT_MUL | 512;
+template <int GROUP, int SOFT = kSoftMul, class R>
 __host__ __device__ __forceinline__ R mulx(R a, R b) {
-  if constexpr ((FV2D_SOFT_MUL >> (GROUP - 1)) & 1) return fv_mul(a, b);
+  if constexpr ((SOFT >> (GROUP - 1)) & 1) return fv_mul(a, b);
   else return a * b;
 }
 
 // {x0 y0, x1 y1} of one group: on the integer pipes in one call
-template <int GROUP>
-__device__ __forceinline__ void mulx2(double x0, double y0, double x1, double y1, double &r0, double &r1) {
-  if constexpr ((FV2D_SOFT_MUL >> (GROUP - 1)) & 1) {
+template <int GROUP, int SOFT = kSoftMul, class R>
+__host__ __device__ __forceinline__ void mulx2(R x0, R y0, R x1, R y1, R &r0, R &r1) {
+#ifdef __CUDA_ARCH__
+  if constexpr (sizeof(R) == 8 && ((SOFT >> (GROUP - 1)) & 1)) {
     const double2 r = softfp::mul2_rn(x0, y0, x1, y1);
     r0 = r.x;
     r1 = r.y;
-  } else {
-    r0 = x0 * y0;
-    r1 = x1 * y1;
+    return;
   }
+#endif
+  r0 = x0 * y0;
+  r1 = x1 * y1;
+}
+// {a1 / b1, a2 / b2}; {a1 / b, a2 / b} with b's reciprocal word r
+__host__ __device__ __forceinline__ void fv_quot2(double a1, double b1, double a2, double b2, double &q1, double &q2) {
+#ifdef __CUDA_ARCH__
+  const double2 q = softfp::quot2_rn(a1, b1, a2, b2);
+  q1 = q.x;
+  q2 = q.y;
+#else
+  q1 = a1 / b1;
+  q2 = a2 / b2;
+#endif
+}
+__host__ __device__ __forceinline__ void fv_quot2(float a1, float b1, float a2, float b2, float &q1, float &q2) {
+  q1 = a1 / b1;
+  q2 = a2 / b2;
+}
+__host__ __device__ __forceinline__ void fv_div2_by(double a1, double a2, double b, uint32_t r, double &q1, double &q2) {
+#ifdef __CUDA_ARCH__
+  const double2 q = softfp::div2_by(a1, a2, b, r);
+  q1 = q.x;
+  q2 = q.y;
+#else
+  (void)r;
+  q1 = a1 / b;
+  q2 = a2 / b;
+#endif
+}
+__host__ __device__ __forceinline__ void fv_div2_by(float a1, float a2, float b, uint32_t, float &q1, float &q2) {
+  q1 = a1 / b;
+  q2 = a2 / b;
 }
 
 enum { IR = 0, IU = 1, IV = 2, IP = 3, IE = 3 };
@@ -195,13 +228,15 @@ __host__ __device__ __forceinline__ S4<R> prim_to_cons(const S4<R> &q, const Gas
 }
 
 // States.h:32-43
-template <class R>
+template <int SOFT = kSoftMul, class R>
 __host__ __device__ __forceinline__ S4<R> cons_to_prim(const S4<R> &u, const Gas<R> &g) {
   S4<R> q;
   q.r = u.r;
   fv_div2(u.u, u.v, u.r, q.u, q.v);
-  R Ek = mulx<4>(fv_half(q.r), mulx<4>(q.u, q.u) + mulx<4>(q.v, q.v));
-  q.p = mulx<4>(u.p - Ek, g.gm1);
+  R uu, vv;
+  mulx2<4, SOFT>(q.u, q.u, q.v, q.v, uu, vv);
+  R Ek = mulx<4, SOFT>(fv_half(q.r), uu + vv);
+  q.p = mulx<4, SOFT>(u.p - Ek, g.gm1);
   return q;
 }
 
@@ -211,14 +246,14 @@ __device__ __forceinline__ R dsqrt(R x) {
 }
 
 // States.h:45-46
-template <class R>
+template <int SOFT = kSoftMul, class R>
 __device__ __forceinline__ R sound_speed(const S4<R> &q, const Gas<R> &g) {
-  return dsqrt(fv_div(mulx<1>(q.p, g.gamma), q.r));
+  return dsqrt(fv_div(mulx<1, SOFT>(q.p, g.gamma), q.r));
 }
 // the same with the reciprocal of q.r already formed (fv_recip)
-template <class R>
+template <int SOFT = kSoftMul, class R>
 __device__ __forceinline__ R sound_speed_r(const S4<R> &q, const Gas<R> &g, uint32_t rr) {
-  return dsqrt(fv_div_by(mulx<1>(q.p, g.gamma), q.r, rr));
+  return dsqrt(fv_div_by(mulx<1, SOFT>(q.p, g.gamma), q.r, rr));
 }
 
 // Update.h:77-85
@@ -235,7 +270,7 @@ __device__ __forceinline__ R sel(bool c, R a, R b) {
 
 // RiemannSolvers.h:7-51.  All three candidates are evaluated, then selected
 // in the reference's branch order (SL >= 0, SR <= 0, else the HLL state).
-template <bool SOFT_AVERAGE = false, class R>
+template <class R>
 __device__ __forceinline__ void riemann_hll(const S4<R> &qL, const S4<R> &qR, S4<R> &f, R &pout, const Gas<R> &g) {
   // every quotient by rho_L (rho_R) shares one reciprocal
   const uint32_t rL = fv_recip(qL.r), rR = fv_recip(qR.r);
@@ -262,16 +297,65 @@ __device__ __forceinline__ void riemann_hll(const S4<R> &qL, const S4<R> &qR, S4
   const R mvL = mulx<9>(qL.r, qL.v), mvR = mulx<9>(qR.r, qR.v);
   const R uEL = (fv_div_by(fv_half(mulx<9>(ruL, ruL) + mulx<9>(mvL, mvL)), qL.r, rL) + peL);
   const R uER = (fv_div_by(fv_half(mulx<9>(ruR, ruR) + mulx<9>(mvR, mvR)), qR.r, rR) + peR);
-  auto avg = [](R a, R b) { return SOFT_AVERAGE ? fv_mul(a, b) : mulx<10>(a, b); };
-  const R SLSR = avg(SL, SR);
+  const R SLSR = mulx<10>(SL, SR);
   const R den = SR - SL;
   const uint32_t rden = fv_recip(den);
   S4<R> FM;
-  FM.r = fv_div_by(avg(SR, FL.r) - avg(SL, FR.r) + avg(SLSR, qR.r - qL.r), den, rden);
-  FM.u = fv_div_by(avg(SR, FL.u) - avg(SL, FR.u) + avg(SLSR, ruR - ruL), den, rden);
-  FM.v = fv_div_by(avg(SR, FL.v) - avg(SL, FR.v) + avg(SLSR, mvR - mvL), den, rden);
-  FM.p = fv_div_by(avg(SR, FL.p) - avg(SL, FR.p) + avg(SLSR, uER - uEL), den, rden);
+  FM.r = fv_div_by(mulx<10>(SR, FL.r) - mulx<10>(SL, FR.r) + mulx<10>(SLSR, qR.r - qL.r), den, rden);
+  FM.u = fv_div_by(mulx<10>(SR, FL.u) - mulx<10>(SL, FR.u) + mulx<10>(SLSR, ruR - ruL), den, rden);
+  FM.v = fv_div_by(mulx<10>(SR, FL.v) - mulx<10>(SL, FR.v) + mulx<10>(SLSR, mvR - mvL), den, rden);
+  FM.p = fv_div_by(mulx<10>(SR, FL.p) - mulx<10>(SL, FR.p) + mulx<10>(SLSR, uER - uEL), den, rden);
   const R pM = fv_half(qL.p + qR.p);
+  const bool left = fv_ge0(SL);
+  const bool right = !left && fv_le0(SR);
+  f.r = left ? FL.r : (right ? FR.r : FM.r);
+  f.u = left ? FL.u : (right ? FR.u : FM.u);
+  f.v = left ? FL.v : (right ? FR.v : FM.v);
+  f.p = left ? FL.p : (right ? FR.p : FM.p);
+  pout = left ? qL.p : (right ? qR.p : pM);
+}
+
+// The same in binary64, its independent products, quotients and sound speeds
+// taken in pairs (one call and two chains each).
+template <int SOFT = kSoftMul>
+__device__ __forceinline__ void riemann_hll(const S4<double> &qL, const S4<double> &qR, S4<double> &f, double &pout,
+                                            const Gas<double> &g) {
+  const double2 c = softfp::sound2(qL.p, qL.r, qR.p, qR.r, g.gamma);
+  const double SL = fv_fmin(qL.u - c.x, qR.u - c.y);
+  const double SR = fv_fmax(qL.u + c.x, qR.u + c.y);
+  double peL, peR, uuL, vvL, uuR, vvR, EkL, EkR, EL, ER;
+  fv_div2_by(qL.p, qR.p, g.gm1, g.rgm1, peL, peR);
+  mulx2<9, SOFT>(qL.u, qL.u, qL.v, qL.v, uuL, vvL);
+  mulx2<9, SOFT>(qR.u, qR.u, qR.v, qR.v, uuR, vvR);
+  mulx2<9, SOFT>(fv_half(qL.r), uuL + vvL, fv_half(qR.r), uuR + vvR, EkL, EkR);
+  EL = peL + EkL;
+  ER = peR + EkR;
+  S4<double> FL, FR;
+  double a, b, mvL, mvR;
+  mulx2<9, SOFT>(qL.r, qL.u, qR.r, qR.u, FL.r, FR.r);
+  mulx2<9, SOFT>(FL.r, qL.u, FR.r, qR.u, a, b);
+  FL.u = a + qL.p;
+  FR.u = b + qR.p;
+  mulx2<9, SOFT>(FL.r, qL.v, FR.r, qR.v, FL.v, FR.v);
+  mulx2<9, SOFT>(qL.p + EL, qL.u, qR.p + ER, qR.u, FL.p, FR.p);
+  mulx2<9, SOFT>(qL.r, qL.v, qR.r, qR.v, mvL, mvR);
+  mulx2<9, SOFT>(FL.r, FL.r, mvL, mvL, uuL, vvL);
+  mulx2<9, SOFT>(FR.r, FR.r, mvR, mvR, uuR, vvR);
+  double wL, wR;
+  fv_quot2(fv_half(uuL + vvL), qL.r, fv_half(uuR + vvR), qR.r, wL, wR);
+  const double duE = (wR + peR) - (wL + peL);
+  const double SLSR = mulx<10, SOFT>(SL, SR);
+  const double den = SR - SL;
+  const uint32_t rden = fv_recip(den);
+  auto average = [&](double fL, double fR, double du) {
+    double x, y;
+    mulx2<10, SOFT>(SR, fL, SL, fR, x, y);
+    return x - y + mulx<10, SOFT>(SLSR, du);
+  };
+  S4<double> FM;
+  fv_div2_by(average(FL.r, FR.r, qR.r - qL.r), average(FL.u, FR.u, FR.r - FL.r), den, rden, FM.r, FM.u);
+  fv_div2_by(average(FL.v, FR.v, mvR - mvL), average(FL.p, FR.p, duE), den, rden, FM.v, FM.p);
+  const double pM = fv_half(qL.p + qR.p);
   const bool left = fv_ge0(SL);
   const bool right = !left && fv_le0(SR);
   f.r = left ? FL.r : (right ? FR.r : FM.r);
@@ -342,6 +426,7 @@ __device__ __forceinline__ double negated_difference(double x) {
 //   - S_K - u_K and rho_K (S_K - u_K) of the star state are the negated (left)
 //     or the same (right) difference and product of the wave speeds' step;
 //   - the total energy is formed for the side the flux is taken from only.
+template <int SOFT = kSoftMul>
 __device__ __forceinline__ void riemann_hllc(const S4<double> &qL, const S4<double> &qR, S4<double> &f, double &pout,
                                              const Gas<double> &g) {
   const double rL = qL.r, uL = qL.u, vL = qL.v, pL = qL.p;
@@ -351,11 +436,11 @@ __device__ __forceinline__ void riemann_hllc(const S4<double> &qL, const S4<doub
   const double SL = um.x - cmax, SR = um.y + cmax;
   const double dL = uL - SL, dR = SR - uR;
   double rcL, rcR, a, b, c, d;
-  mulx2<5>(rL, dL, rR, dR, rcL, rcR);
-  mulx2<1>(rcR, uR, rcL, uL, a, b);
-  mulx2<6>(rcR, pL, rcL, pR, c, d);
+  mulx2<5, SOFT>(rL, dL, rR, dR, rcL, rcR);
+  mulx2<1, SOFT>(rcR, uR, rcL, uL, a, b);
+  mulx2<6, SOFT>(rcR, pL, rcL, pR, c, d);
   double uS, pS;
-  fv_div2(a + b + (pL - pR), c + d + mulx<6>(mulx<6>(rcL, rcR), uL - uR), rcR + rcL, uS, pS);
+  fv_div2(a + b + (pL - pR), c + d + mulx<6, SOFT>(mulx<6, SOFT>(rcL, rcR), uL - uR), rcR + rcL, uS, pS);
   const bool sideL = fv_gt0(uS);
   // branch order of RiemannSolvers.h:89-112
   const bool bL = fv_gt0(SL);
@@ -369,18 +454,18 @@ __device__ __forceinline__ void riemann_hllc(const S4<double> &qL, const S4<doub
   const double dK = left ? negated_difference(dL) : dR;   // S_K - u_K
   const double rcK = left ? negated_difference(rcL) : rcR;  // rho_K (S_K - u_K)
   double E;
-  mulx2<1>(su, su, sv, sv, a, b);
-  mulx2<2>(fv_half(sr), a + b, sp, g.entho, c, d);
+  mulx2<1, SOFT>(su, su, sv, sv, a, b);
+  mulx2<2, SOFT>(fv_half(sr), a + b, sp, g.entho, c, d);
   E = c + d;
   double rS, ES;
-  mulx2<7>(dK, E, sp, su, a, b);
-  fv_div2(rcK, a - b + mulx<7>(pS, uS), SK - uS, rS, ES);
+  mulx2<7, SOFT>(dK, E, sp, su, a, b);
+  fv_div2(rcK, a - b + mulx<7, SOFT>(pS, uS), SK - uS, rS, ES);
   if (bStar) {
     sr = rS; su = uS; sp = pS; E = ES;
   }
   pout = sp;
-  mulx2<1>(sr, su, E + sp, su, f.r, f.p);
-  mulx2<1>(f.r, su, f.r, sv, a, f.v);
+  mulx2<1, SOFT>(sr, su, E + sp, su, f.r, f.p);
+  mulx2<1, SOFT>(f.r, su, f.r, sv, a, f.v);
   f.u = a + sp;
 }
 
@@ -414,13 +499,56 @@ __device__ __forceinline__ void riemann_fslp(const S4<R> &qL, const S4<R> &qR, S
   pout = Pi;
 }
 
+// The same in binary64, in pairs as above.
+template <int SOFT = kSoftMul>
+__device__ __forceinline__ void riemann_fslp(const S4<double> &qL, const S4<double> &qR, S4<double> &f, double &pout,
+                                             double gdx, const Gas<double> &g) {
+  const double uL = qL.u, pL = qL.p, uR = qR.u, pR = qR.p;
+  const double2 c = softfp::sound2(pL, qL.r, pR, qR.r, g.gamma);
+  double zL, zR, mL, mR;
+  mulx2<14, SOFT>(qL.r, c.x, qR.r, c.y, zL, zR);
+  const double ai = mulx<14, SOFT>(g.fslp_K, fv_lt(zL, zR) ? zR : zL);
+  fv_quot2(fabs(uL), c.x, fabs(uR), c.y, mL, mR);
+  const double mx = fv_lt(mL, mR) ? mR : mL;
+  const double theta = fv_lt(mx, 1.0) ? mx : 1.0;
+  double a, b, uu, vv, w, z;
+  mulx2<14, SOFT>(fv_half(qL.r + qR.r), gdx, fv_half(theta), ai, a, b);
+  mulx2<14, SOFT>(fv_div(0.5, ai), pR - pL - a, b, uR - uL, a, b);
+  const double ustar = fv_half(uR + uL) - a;
+  const double Pi = fv_half(pR + pL) - b;
+  const bool up = fv_gt0(ustar);
+  const double sr = up ? qL.r : qR.r;
+  const double su = up ? uL : uR;
+  const double sv = up ? qL.v : qR.v;
+  const double sp = up ? pL : pR;
+  mulx2<14, SOFT>(su, su, sv, sv, uu, vv);
+  mulx2<14, SOFT>(fv_half(sr), uu + vv, ustar, sr, w, z);
+  const double Estar = w + fv_div_by(sp, g.gm1, g.rgm1);
+  f.r = z;
+  mulx2<14, SOFT>(z, su, z, sv, a, f.v);
+  f.u = a + Pi;
+  f.p = mulx<14, SOFT>(ustar, Estar + Pi);
+  pout = Pi;
+}
+
 enum { RS_HLL = 0, RS_HLLC = 1, RS_FSLP = 2 };
 
-// VISC: the caller is a viscous kernel (which products run on which pipe)
-template <int RS, bool VISC = false, class R>
-__device__ __forceinline__ void riemann(const S4<R> &qL, const S4<R> &qR, S4<R> &f, R &pout, R gdx, const Gas<R> &g) {
+// SOFT: which products run on the integer pipes (binary64)
+template <int RS, int SOFT = kSoftMul>
+__device__ __forceinline__ void riemann(const S4<double> &qL, const S4<double> &qR, S4<double> &f, double &pout,
+                                        double gdx, const Gas<double> &g) {
   if constexpr (RS == RS_HLL)
-    riemann_hll<VISC>(qL, qR, f, pout, g);
+    riemann_hll<SOFT>(qL, qR, f, pout, g);
+  else if constexpr (RS == RS_FSLP)
+    riemann_fslp<SOFT>(qL, qR, f, pout, gdx, g);
+  else
+    riemann_hllc<SOFT>(qL, qR, f, pout, g);
+}
+template <int RS>
+__device__ __forceinline__ void riemann(const S4<float> &qL, const S4<float> &qR, S4<float> &f, float &pout, float gdx,
+                                        const Gas<float> &g) {
+  if constexpr (RS == RS_HLL)
+    riemann_hll(qL, qR, f, pout, g);
   else if constexpr (RS == RS_FSLP)
     riemann_fslp(qL, qR, f, pout, gdx, g);
   else
@@ -430,16 +558,16 @@ __device__ __forceinline__ void riemann(const S4<R> &qL, const S4<R> &qR, S4<R> 
 // Extension (no reference counterpart): primitive-variable MUSCL-Hancock
 // half-step qh = q - (dt/2dx) A(q) sx - (dt/2dy) B(q) sy, with ax = 0.5 dt/dx,
 // ay = 0.5 dt/dy and sx, sy the full minmod slopes.
-template <class R>
+template <int SOFT = kSoftMul, class R>
 __host__ __device__ __forceinline__ S4<R> hancock(const S4<R> &q, const S4<R> &sx, const S4<R> &sy, R ax, R ay,
                                                   R gamma) {
   S4<R> h;
-  h.r = q.r - (mulx<13>(ax, mulx<13>(q.u, sx.r) + mulx<13>(q.r, sx.u)) +
-               mulx<13>(ay, mulx<13>(q.v, sy.r) + mulx<13>(q.r, sy.v)));
-  h.u = q.u - (mulx<13>(ax, mulx<13>(q.u, sx.u) + fv_div(sx.p, q.r)) + mulx<13>(ay, mulx<13>(q.v, sy.u)));
-  h.v = q.v - (mulx<13>(ax, mulx<13>(q.u, sx.v)) + mulx<13>(ay, mulx<13>(q.v, sy.v) + fv_div(sy.p, q.r)));
-  h.p = q.p - (mulx<13>(ax, mulx<13>(mulx<13>(gamma, q.p), sx.u) + mulx<13>(q.u, sx.p)) +
-               mulx<13>(ay, mulx<13>(mulx<13>(gamma, q.p), sy.v) + mulx<13>(q.v, sy.p)));
+  h.r = q.r - (mulx<13, SOFT>(ax, mulx<13, SOFT>(q.u, sx.r) + mulx<13, SOFT>(q.r, sx.u)) +
+               mulx<13, SOFT>(ay, mulx<13, SOFT>(q.v, sy.r) + mulx<13, SOFT>(q.r, sy.v)));
+  h.u = q.u - (mulx<13, SOFT>(ax, mulx<13, SOFT>(q.u, sx.u) + fv_div(sx.p, q.r)) + mulx<13, SOFT>(ay, mulx<13, SOFT>(q.v, sy.u)));
+  h.v = q.v - (mulx<13, SOFT>(ax, mulx<13, SOFT>(q.u, sx.v)) + mulx<13, SOFT>(ay, mulx<13, SOFT>(q.v, sy.v) + fv_div(sy.p, q.r)));
+  h.p = q.p - (mulx<13, SOFT>(ax, mulx<13, SOFT>(mulx<13, SOFT>(gamma, q.p), sx.u) + mulx<13, SOFT>(q.u, sx.p)) +
+               mulx<13, SOFT>(ay, mulx<13, SOFT>(mulx<13, SOFT>(gamma, q.p), sy.v) + mulx<13, SOFT>(q.v, sy.p)));
   return h;
 }
 

@@ -208,9 +208,28 @@ FV2D_SF_CALL double2 div2_rn(double a1, double a2, double b) {
   return make_double2(div_core(bits(a1), bits(b), x), div_core(bits(a2), bits(b), x));
 }
 
+// {a1 / b1, a2 / b2} in one call
+FV2D_SF_CALL double2 quot2_rn(double a1, double b1, double a2, double b2) {
+  Range r;
+  r.add(bits(a1));
+  r.add(bits(b1));
+  r.add(bits(a2));
+  r.add(bits(b2));
+  if (!r.ok()) return make_double2(div_with(a1, b1, recip_of(b1)), div_with(a2, b2, recip_of(b2)));
+  return make_double2(div_core(bits(a1), bits(b1), recip_of(b1)), div_core(bits(a2), bits(b2), recip_of(b2)));
+}
+
 // Quotients by one divisor b: recip_of(b) forms its reciprocal word once,
 // div_by(a, b, x) each quotient.
 FV2D_SF_CALL double div_by(double a, double b, uint32_t x) { return div_with(a, b, x); }
+FV2D_SF_CALL double2 div2_by(double a1, double a2, double b, uint32_t x) {
+  Range r;
+  r.add(bits(a1));
+  r.add(bits(a2));
+  r.add(bits(b));
+  if (!r.ok()) return make_double2(div_with(a1, b, x), div_with(a2, b, x));
+  return make_double2(div_core(bits(a1), bits(b), x), div_core(bits(a2), bits(b), x));
+}
 
 // recip_of(b) for a divisor known on the host (the mesh spacings): 2^83 / mb
 // rounded down.
@@ -393,13 +412,12 @@ FV2D_SF double mul_pow2(double x, double y, int k) {
 // x * 0.5
 FV2D_SF double half(double x) { return mul_pow2(x, 0.5, -1); }
 
-// sqrt(fmax_nm(gamma pL / rL, gamma pR / rR)), each operation rounded: the
-// larger sound speed of two states, in one call with two independent chains.
-// Positive operands of that range keep every intermediate normal.
-FV2D_SF_CALL double sound_max_rare(double pL, double rL, double pR, double rR, double gamma) {
-  return sqrt_rn(fmax_nm(div_rn(mul_rn(pL, gamma), rL), div_rn(mul_rn(pR, gamma), rR)));
-}
-FV2D_SF_CALL double sound_max(double pL, double rL, double pR, double rR, double gamma) {
+// The sound speeds of two states, sqrt(gamma p / r) with each operation
+// rounded, in one call with two independent chains: both of them
+// (sound2), or the larger one (sound_max: the square root of the larger
+// quotient, a correctly rounded square root being monotone).  Positive
+// operands of the common range keep every intermediate normal.
+FV2D_SF bool sound_range(double pL, double rL, double pR, double rR, double gamma) {
   Range r;
   r.add(bits(pL));
   r.add(bits(rL));
@@ -407,10 +425,24 @@ FV2D_SF_CALL double sound_max(double pL, double rL, double pR, double rR, double
   r.add(bits(rR));
   r.add(bits(gamma));
   const uint32_t signs = hi32(bits(pL)) | hi32(bits(rL)) | hi32(bits(pR)) | hi32(bits(rR)) | hi32(bits(gamma));
-  if (!r.ok() || (int32_t)signs < 0) return sound_max_rare(pL, rL, pR, rR, gamma);
-  const uint64_t a = bits(div_core(bits(mul_core(bits(gamma), bits(pL))), bits(rL), recip_of(rL)));
-  const uint64_t b = bits(div_core(bits(mul_core(bits(gamma), bits(pR))), bits(rR), recip_of(rR)));
+  return r.ok() && (int32_t)signs >= 0;
+}
+FV2D_SF uint64_t sound_quotient(double p, double r, double gamma) {
+  return bits(div_core(bits(mul_core(bits(gamma), bits(p))), bits(r), recip_of(r)));
+}
+FV2D_SF_CALL double sound_max_rare(double pL, double rL, double pR, double rR, double gamma) {
+  return sqrt_rn(fmax_nm(div_rn(mul_rn(pL, gamma), rL), div_rn(mul_rn(pR, gamma), rR)));
+}
+FV2D_SF_CALL double sound_max(double pL, double rL, double pR, double rR, double gamma) {
+  if (!sound_range(pL, rL, pR, rR, gamma)) return sound_max_rare(pL, rL, pR, rR, gamma);
+  const uint64_t a = sound_quotient(pL, rL, gamma), b = sound_quotient(pR, rR, gamma);
   return sqrt_core(a > b ? a : b);
+}
+FV2D_SF_CALL double sound_rare(double p, double r, double gamma) { return sqrt_rn(div_rn(mul_rn(p, gamma), r)); }
+FV2D_SF_CALL double2 sound2(double pL, double rL, double pR, double rR, double gamma) {
+  if (!sound_range(pL, rL, pR, rR, gamma))
+    return make_double2(sound_rare(pL, rL, gamma), sound_rare(pR, rR, gamma));
+  return make_double2(sqrt_core(sound_quotient(pL, rL, gamma)), sqrt_core(sound_quotient(pR, rR, gamma)));
 }
 
 }  // namespace softfp

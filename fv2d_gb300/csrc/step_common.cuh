@@ -8,13 +8,20 @@
 
 namespace fv2d {
 
-// Tile of interior cells owned by one CTA of the fused step kernel.
-constexpr int TX = 16;  // cells along x (even: TMA rows start on 16-byte boundaries)
-constexpr int TY = 16;  // cells along y
 constexpr int HALO = 2; // ghost depth read by PLM + the 3x3 viscous stencil
-constexpr int SW = TX + 2 * HALO;  // staged tile width  (TMA box x)
-constexpr int SH = TY + 2 * HALO;  // staged tile height (TMA box y)
-constexpr int NT = 288;            // threads per CTA (9 warps: the 544 faces of a tile in two rounds)
+
+// Tile of interior cells owned by one CTA of the fused step kernel.
+template <int TX_, int TY_, int NT_>
+struct Tile {
+  static constexpr int TX = TX_;             // cells along x (even: TMA rows start on 16-byte boundaries)
+  static constexpr int TY = TY_;             // cells along y
+  static constexpr int SW = TX + 2 * HALO;   // staged tile width  (TMA box x)
+  static constexpr int SH = TY + 2 * HALO;   // staged tile height (TMA box y)
+  static constexpr int NT = NT_;             // threads per CTA
+};
+using WideTile = Tile<16, 16, 288>;  // 9 warps: the 544 faces of a tile in two rounds
+using SmallTile = Tile<8, 8, 160>;   // 5 warps: the 144 faces of a tile in one round
+enum { TILE_WIDE = 0, TILE_SMALL = 1 };
 
 enum { RECON_PCM = 0, RECON_PLM = 2, RECON_MH = 3 };
 enum { STAGE_EULER = 0, STAGE_RK2_PREDICT = 1, STAGE_RK2_CORRECT = 2 };

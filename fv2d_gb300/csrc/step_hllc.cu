@@ -1,50 +1,11 @@
 // step_hllc.cu -- instantiations of the fused FP64 step for the HLLC solver
 // (one translation unit per solver so that they compile in parallel).
-#include "step_kernel.cuh"
+#include "step_launch.cuh"
 
 namespace fv2d {
-
-namespace {
-template <int RECON, bool VISC>
-cudaError_t attr() {
-  return cudaFuncSetAttribute(step_kernel<RECON, RS_HLLC, VISC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)Smem<RECON, VISC>::BYTES);
+cudaError_t set_step_attrs_hllc() { return set_step_attrs<RS_HLLC>(); }
+cudaError_t launch_step_hllc(int tile, int recon, dim3 grid, cudaStream_t s, const CUtensorMap &t0,
+                            const CUtensorMap &t1, const StepArgs &a) {
+  return launch_step_rs<RS_HLLC>(tile, recon, grid, s, t0, t1, a);
 }
-template <bool VISC>
-void launch(int recon, dim3 grid, cudaStream_t s, const CUtensorMap &t0, const CUtensorMap &t1, const StepArgs &a) {
-  switch (recon) {
-    case RECON_PLM:
-      step_kernel<RECON_PLM, RS_HLLC, VISC><<<grid, NT, Smem<RECON_PLM, VISC>::BYTES, s>>>(t0, t1, a);
-      break;
-    case RECON_MH:
-      step_kernel<RECON_MH, RS_HLLC, VISC><<<grid, NT, Smem<RECON_MH, VISC>::BYTES, s>>>(t0, t1, a);
-      break;
-    default:
-      step_kernel<RECON_PCM, RS_HLLC, VISC><<<grid, NT, Smem<RECON_PCM, VISC>::BYTES, s>>>(t0, t1, a);
-      break;
-  }
-}
-}  // namespace
-
-cudaError_t set_step_attrs_hllc() {
-  cudaError_t e = attr<RECON_PCM, false>();
-  if (e == cudaSuccess) e = attr<RECON_PLM, false>();
-  if (e == cudaSuccess) e = attr<RECON_MH, false>();
-  if (e == cudaSuccess) e = attr<RECON_PCM, true>();
-  if (e == cudaSuccess) e = attr<RECON_PLM, true>();
-  if (e == cudaSuccess) e = attr<RECON_MH, true>();
-  return e;
-}
-
-// the viscous terms are a separate instantiation: kernels without them keep
-// their registers and shared memory
-cudaError_t launch_step_hllc(int recon, dim3 grid, cudaStream_t s, const CUtensorMap &t0, const CUtensorMap &t1,
-                            const StepArgs &a) {
-  if (a.visc)
-    launch<true>(recon, grid, s, t0, t1, a);
-  else
-    launch<false>(recon, grid, s, t0, t1, a);
-  return cudaGetLastError();
-}
-
 }  // namespace fv2d

@@ -119,41 +119,56 @@ __device__ __forceinline__ bool gidx_ok(long long i, long long n, int *err) {
 
 // Shared-memory layout (in doubles) for a reconstruction type, with or
 // without the viscous face terms.
-template <int RECON, bool VISC = false>
+template <class T_, int RECON, bool VISC = false>
 struct Smem {
+  static constexpr int TX = T_::TX, TY = T_::TY;
   static constexpr int R1W = TX + 2, R1H = TY + 2;  // tile + 1-cell ring
   static constexpr int R1 = R1W * R1H;
   static constexpr int Q = 0;
-  static constexpr int SX = Q + 4 * SH * SW;
+  static constexpr int SX = Q + 4 * T_::SH * T_::SW;
   static constexpr int SY = SX + ((RECON != RECON_PCM) ? 4 * R1 : 0);
   static constexpr int QH = SY + ((RECON != RECON_PCM) ? 4 * R1 : 0);
   static constexpr int FX = QH + ((RECON == RECON_MH) ? 4 * R1 : 0);
   static constexpr int FY = FX + 4 * TY * (TX + 1);
   static constexpr int PY = FY + 4 * (TY + 1) * TX;
-  static constexpr int T = PY + (TY + 1) * TX;
+  // the neighbour differences share the face-flux area
+  static constexpr int NDX = 4 * TY * (TX + 3), NDY = 4 * (TY + 3) * TX;
+  static constexpr int FEND = PY + (TY + 1) * TX, DEND = (RECON == RECON_PLM) ? FX + NDX + NDY : 0;
+  static constexpr int T = FEND > DEND ? FEND : DEND;
   static constexpr int VX = T + R1;                                  // viscous x-face terms, 3 x TY x (TX+1)
   static constexpr int VY = VX + (VISC ? 3 * TY * (TX + 1) : 0);     // viscous y-face terms, 3 x (TY+1) x TX
   static constexpr int TOTAL = VY + (VISC ? 3 * (TY + 1) * TX : 0);
   static constexpr size_t BYTES = sizeof(double) * (TOTAL + 1) + 128;  // + spare slot + alignment slack
 };
 
-// CTAs per SM: 3.  Without viscosity, measured faster with more at the price
+// CTAs per SM: 5 of the small tile; 3 of the wide one.  Without viscosity, measured faster with more at the price
 // of register spills (their shared memory still fits): PCM with HLL or HLLC
 // at 5 (40 registers), PCM with FSLP and PLM with HLL or FSLP at 4 (56); PLM
 // and MUSCL-Hancock with HLLC stay at 3.
-template <int RECON, int RS>
+template <class T_, int RECON, int RS>
 constexpr int step_ctas_per_sm(bool visc) {
+  if (T_::TX < 16) return 5;
   if (visc) return 3;
   if (RECON == RECON_PCM) return RS == RS_FSLP ? 4 : 5;
   if (RECON == RECON_PLM && RS != RS_HLLC) return 4;
   return 3;
 }
 
-template <int RECON, int RS, bool VISC>
-__global__ void __launch_bounds__(NT, step_ctas_per_sm<RECON, RS>(VISC))
+// The products on the integer pipes (physics.cuh): none on small grids, where
+// no pipe is full and a hardware product's latency is a fifth of the
+// integer-pipe one's (Sod 512 x 8: 20.5 -> 18.0 us a step).
+template <class T_>
+__host__ __device__ constexpr int step_soft_mul(bool visc) {
+  return T_::TX < 16 ? 0 : visc ? kSoftMulVisc : kSoftMul;
+}
+
+template <class T_, int RECON, int RS, bool VISC>
+__global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
     step_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant__ CUtensorMap tmQ1,
                 const StepArgs a) {
-  using L = Smem<RECON, VISC>;
+  using L = Smem<T_, RECON, VISC>;
+  constexpr int TX = T_::TX, TY = T_::TY, SW = T_::SW, SH = T_::SH, NT = T_::NT;
+  constexpr int SOFT = step_soft_mul<T_>(VISC);
   // Aligned by offsetting the shared array itself (not through an integer
   // round trip, which would turn every tile access into a generic load).
   extern __shared__ __align__(128) unsigned char fv2d_step_smem[];
@@ -174,6 +189,7 @@ __global__ void __launch_bounds__(NT, step_ctas_per_sm<RECON, RS>(VISC))
 
   const int bx = blockIdx.x, by = blockIdx.y;
   const int i0 = bx * TX, j0 = by * TY;  // first interior cell of the tile
+  const int nx = min(TX, a.Nx - i0), ny = min(TY, a.Ny - j0);  // its cells inside the grid
 
   // ---- 1. stage tile + halo (padded coordinates start at the halo) -------
   if (tid == 0) {
@@ -204,8 +220,7 @@ __global__ void __launch_bounds__(NT, step_ctas_per_sm<RECON, RS>(VISC))
     // the next: Update.h:70-76 computes both), held in the face-flux area
     // until the Riemann pass: DX[k][r][f] = Q(f+1) - Q(f) on padded row r+2,
     // DY[k][g][c] = Q(g+1) - Q(g) on padded column c+2.
-    constexpr int NDX = 4 * TY * (TX + 3), NDY = 4 * (TY + 3) * TX;
-    static_assert(NDX + NDY <= L::T - L::FX, "difference arrays exceed the face-flux area");
+    constexpr int NDX = L::NDX, NDY = L::NDY;
     // DX at L::FX, DY at L::FX + NDX
     for (int it = tid; it < NDX + NDY; it += NT) {
       if (it < NDX) {
@@ -255,6 +270,7 @@ __global__ void __launch_bounds__(NT, step_ctas_per_sm<RECON, RS>(VISC))
   if (a.tc) {
     for (int it = tid; it < L::R1; it += NT) {
       const int ly = it / L::R1W + 1, lx = it % L::R1W + 1;
+      if (ly > ny + 2 || lx > nx + 2) continue;  // past the grid's ghost ring
       sR1(L::T, 0, ly, lx) = fv_div(sQ(3, ly, lx), sQ(0, ly, lx));
     }
     if (tid == NT - 1) {
@@ -267,9 +283,10 @@ __global__ void __launch_bounds__(NT, step_ctas_per_sm<RECON, RS>(VISC))
     const double ax = fv_div(0.5 * dt, a.dx), ay = fv_div(0.5 * dt, a.dy);
     for (int it = tid; it < L::R1; it += NT) {
       const int ly = it / L::R1W + 1, lx = it % L::R1W + 1;
+      if (ly > ny + 2 || lx > nx + 2) continue;  // past the grid's ghost ring
       S4<double> sx{sR1(L::SX, 0, ly, lx), sR1(L::SX, 1, ly, lx), sR1(L::SX, 2, ly, lx), sR1(L::SX, 3, ly, lx)};
       S4<double> sy{sR1(L::SY, 0, ly, lx), sR1(L::SY, 1, ly, lx), sR1(L::SY, 2, ly, lx), sR1(L::SY, 3, ly, lx)};
-      S4<double> h = hancock(cellQ(ly, lx), sx, sy, ax, ay, a.gamma);
+      S4<double> h = hancock<SOFT>(cellQ(ly, lx), sx, sy, ax, ay, a.gamma);
       sR1(L::QH, 0, ly, lx) = h.r;
       sR1(L::QH, 1, ly, lx) = h.u;
       sR1(L::QH, 2, ly, lx) = h.v;
@@ -315,6 +332,8 @@ __global__ void __launch_bounds__(NT, step_ctas_per_sm<RECON, RS>(VISC))
         c = g % TX;
         lyR = r + 2; lxR = c + 2; lyL = lyR - 1; lxL = lxR;
       }
+      // faces past the grid's edge (a ragged tile) bound no cell
+      if (r >= ny + ydir || c >= nx + !ydir) continue;
       S4<double> qL = face_state(lyL, lxL, true, ydir);
       S4<double> qR = face_state(lyR, lxR, false, ydir);
       if (ydir) {  // swap_component (States.h:103-110)
@@ -323,7 +342,7 @@ __global__ void __launch_bounds__(NT, step_ctas_per_sm<RECON, RS>(VISC))
       }
       S4<double> fl;
       double pout;
-      riemann<RS, VISC>(qL, qR, fl, pout, ydir ? a.gy_dy : a.gx_dx, gas);
+      riemann<RS, SOFT>(qL, qR, fl, pout, ydir ? a.gy_dy : a.gx_dx, gas);
       if (!ydir) {
         const int F = L::FX + r * (TX + 1) + c;
         SMI(F) = fl.r;
@@ -358,15 +377,15 @@ __global__ void __launch_bounds__(NT, step_ctas_per_sm<RECON, RS>(VISC))
         auto V_ = [&](int dj, int x) { return sQ(2, ly + dj, x); };
         const double qiu = fv_half(U_(0, xs) + U_(0, xm));
         const double qiv = fv_half(V_(0, xs) + V_(0, xm));
-        const double dudx = mulx<11>(odx, U_(0, xs) - U_(0, xm));
-        const double dvdx = mulx<11>(odx, V_(0, xs) - V_(0, xm));
-        const double dudy = mulx<11>(q_ody, U_(1, xs) - U_(-1, xs) + U_(1, xm) - U_(-1, xm));
-        const double dvdy = mulx<11>(q_ody, V_(1, xs) - V_(-1, xs) + V_(1, xm) - V_(-1, xm));
-        const double tau_xx = mulx<11>(four_thirds, dudx) - mulx<11>(two_thirds, dvdy);
+        const double dudx = mulx<11, SOFT>(odx, U_(0, xs) - U_(0, xm));
+        const double dvdx = mulx<11, SOFT>(odx, V_(0, xs) - V_(0, xm));
+        const double dudy = mulx<11, SOFT>(q_ody, U_(1, xs) - U_(-1, xs) + U_(1, xm) - U_(-1, xm));
+        const double dvdy = mulx<11, SOFT>(q_ody, V_(1, xs) - V_(-1, xs) + V_(1, xm) - V_(-1, xm));
+        const double tau_xx = mulx<11, SOFT>(four_thirds, dudx) - mulx<11, SOFT>(two_thirds, dvdy);
         const double tau_xy = dvdx + dudy;
-        SMI(L::VX + f) = mulx<11>(mu, tau_xx);
-        SMI(L::VX + f + NVX) = mulx<11>(mu, tau_xy);
-        SMI(L::VX + f + 2 * NVX) = mulx<11>(mu, mulx<11>(tau_xx, qiu) + mulx<11>(tau_xy, qiv));
+        SMI(L::VX + f) = mulx<11, SOFT>(mu, tau_xx);
+        SMI(L::VX + f + NVX) = mulx<11, SOFT>(mu, tau_xy);
+        SMI(L::VX + f + 2 * NVX) = mulx<11, SOFT>(mu, mulx<11, SOFT>(tau_xx, qiu) + mulx<11, SOFT>(tau_xy, qiv));
       } else {  // between rows r+1 (s-1) and r+2 (s) of column c+2
         const int g = f - NVX;
         const int r = g / TX, c = g % TX;
@@ -375,15 +394,15 @@ __global__ void __launch_bounds__(NT, step_ctas_per_sm<RECON, RS>(VISC))
         auto V_ = [&](int y, int di) { return sQ(2, y, lx + di); };
         const double qiu = fv_half(U_(ys, 0) + U_(ym, 0));
         const double qiv = fv_half(V_(ys, 0) + V_(ym, 0));
-        const double dudy = mulx<11>(ody, U_(ys, 0) - U_(ym, 0));
-        const double dvdy = mulx<11>(ody, V_(ys, 0) - V_(ym, 0));
-        const double dudx = mulx<11>(q_odx, U_(ys, 1) - U_(ys, -1) + U_(ym, 1) - U_(ym, -1));
-        const double dvdx = mulx<11>(q_odx, V_(ys, 1) - V_(ys, -1) + V_(ym, 1) - V_(ym, -1));
-        const double tau_yy = mulx<11>(four_thirds, dvdy) - mulx<11>(two_thirds, dudx);
+        const double dudy = mulx<11, SOFT>(ody, U_(ys, 0) - U_(ym, 0));
+        const double dvdy = mulx<11, SOFT>(ody, V_(ys, 0) - V_(ym, 0));
+        const double dudx = mulx<11, SOFT>(q_odx, U_(ys, 1) - U_(ys, -1) + U_(ym, 1) - U_(ym, -1));
+        const double dvdx = mulx<11, SOFT>(q_odx, V_(ys, 1) - V_(ys, -1) + V_(ym, 1) - V_(ym, -1));
+        const double tau_yy = mulx<11, SOFT>(four_thirds, dvdy) - mulx<11, SOFT>(two_thirds, dudx);
         const double tau_xy = dvdx + dudy;
-        SMI(L::VY + g) = mulx<11>(mu, tau_xy);
-        SMI(L::VY + g + NVY) = mulx<11>(mu, tau_yy);
-        SMI(L::VY + g + 2 * NVY) = mulx<11>(mu, mulx<11>(tau_xy, qiu) + mulx<11>(tau_yy, qiv));
+        SMI(L::VY + g) = mulx<11, SOFT>(mu, tau_xy);
+        SMI(L::VY + g + NVY) = mulx<11, SOFT>(mu, tau_yy);
+        SMI(L::VY + g + 2 * NVY) = mulx<11, SOFT>(mu, mulx<11, SOFT>(tau_xy, qiu) + mulx<11, SOFT>(tau_yy, qiv));
       }
     }
   }
@@ -403,7 +422,7 @@ __global__ void __launch_bounds__(NT, step_ctas_per_sm<RECON, RS>(VISC))
   for (int cidx = tid; cidx < TX * TY; cidx += NT) {
     const int ry = cidx / TX, rx = cidx % TX;
     const int i = i0 + rx, j = j0 + ry;
-    if (i >= a.Nx || j >= a.Ny) continue;
+    if (rx >= nx || ry >= ny) continue;
     const int ly = ry + 2, lx = rx + 2;
     const long long g = (long long)(j + HALO) * P + (i + HALO);
     if (!gok(g, PL)) continue;
@@ -418,8 +437,13 @@ __global__ void __launch_bounds__(NT, step_ctas_per_sm<RECON, RS>(VISC))
       constexpr int S = TY * (TX + 1);
       const double FL0 = SMI(F), FR0 = SMI(F + 1);
 #pragma unroll
-      for (int k = 0; k < 4; ++k)
-        un[k] += ddivc(mulx<3>(SMI(F + k * S) - SMI(F + k * S + 1), dt), a.dx, a.inv_dx, a.dx_pow2, a.rw_dx);
+      for (int k = 0; k < 4; k += 2) {
+        double d0, d1;
+        mulx2<3, SOFT>(SMI(F + k * S) - SMI(F + k * S + 1), dt, SMI(F + (k + 1) * S) - SMI(F + (k + 1) * S + 1), dt,
+                       d0, d1);
+        un[k] += ddivc(d0, a.dx, a.inv_dx, a.dx_pow2, a.rw_dx);
+        un[k + 1] += ddivc(d1, a.dx, a.inv_dx, a.dx_pow2, a.rw_dx);
+      }
       if (a.grav_mode) {
         const double gv = (a.grav_mode == 1) ? a.gxf : (double)a.grav_row[j];
         un[2] += dt * rho * gv;
@@ -449,7 +473,12 @@ __global__ void __launch_bounds__(NT, step_ctas_per_sm<RECON, RS>(VISC))
         }
       }
 #pragma unroll
-      for (int k = 0; k < 4; ++k) un[k] += ddivc(mulx<3>(FL[k] - FR[k], dt), a.dy, a.inv_dy, a.dy_pow2, a.rw_dy);
+      for (int k = 0; k < 4; k += 2) {
+        double d0, d1;
+        mulx2<3, SOFT>(FL[k] - FR[k], dt, FL[k + 1] - FR[k + 1], dt, d0, d1);
+        un[k] += ddivc(d0, a.dy, a.inv_dy, a.dy_pow2, a.rw_dy);
+        un[k + 1] += ddivc(d1, a.dy, a.inv_dy, a.dy_pow2, a.rw_dy);
+      }
       if (a.grav_mode) {
         un[2] += dt * rho * gv;
         un[3] += dt * 0.5 * (FL[0] + FR[0]) * gv;
@@ -462,10 +491,13 @@ __global__ void __launch_bounds__(NT, step_ctas_per_sm<RECON, RS>(VISC))
       const double TU = sR1(L::T, 0, ly - 1, lx), TD = sR1(L::T, 0, ly + 1, lx);
       const double kL = a.kap_row[4 * j + 0], kR = a.kap_row[4 * j + 1];
       const double kU = a.kap_row[4 * j + 2], kD = a.kap_row[4 * j + 3];
-      double FLt = ddivc(mulx<12>(kL, TC - TL), a.dx, a.inv_dx, a.dx_pow2, a.rw_dx);
-      double FRt = ddivc(mulx<12>(kR, TR - TC), a.dx, a.inv_dx, a.dx_pow2, a.rw_dx);
-      const double FUt = ddivc(mulx<12>(kU, TC - TU), a.dy, a.inv_dy, a.dy_pow2, a.rw_dy);
-      const double FDt = ddivc(mulx<12>(kD, TD - TC), a.dy, a.inv_dy, a.dy_pow2, a.rw_dy);
+      double FLt, FRt, FUt, FDt;
+      mulx2<12, SOFT>(kL, TC - TL, kR, TR - TC, FLt, FRt);
+      mulx2<12, SOFT>(kU, TC - TU, kD, TD - TC, FUt, FDt);
+      FLt = ddivc(FLt, a.dx, a.inv_dx, a.dx_pow2, a.rw_dx);
+      FRt = ddivc(FRt, a.dx, a.inv_dx, a.dx_pow2, a.rw_dx);
+      FUt = ddivc(FUt, a.dy, a.inv_dy, a.dy_pow2, a.rw_dy);
+      FDt = ddivc(FDt, a.dy, a.inv_dy, a.dy_pow2, a.rw_dy);
       if (j == 0 && a.bctc_ymin != 0) {
         if (a.bctc_ymin == 1)
           FLt = ddivc(kL * 2.0 * (TC - a.bctc_ymin_value), a.dy, a.inv_dy, a.dy_pow2, a.rw_dy);
@@ -478,7 +510,9 @@ __global__ void __launch_bounds__(NT, step_ctas_per_sm<RECON, RS>(VISC))
         else
           FRt = kR * a.bctc_ymax_value;
       }
-      un[3] += mulx<12>(s_tc[0], FRt - FLt) + mulx<12>(s_tc[1], FDt - FUt);
+      double dx_part, dy_part;
+      mulx2<12, SOFT>(s_tc[0], FRt - FLt, s_tc[1], FDt - FUt, dx_part, dy_part);
+      un[3] += dx_part + dy_part;
     }
     // viscosity (Viscosity.h:63-107): the face terms of the face pass, the
     // -side face negated, accumulated in the reference's order
@@ -500,9 +534,11 @@ __global__ void __launch_bounds__(NT, step_ctas_per_sm<RECON, RS>(VISC))
       fy2 += SMI(Vn + NVY + TX);
       fy3 += SMI(Vn + 2 * NVY + TX);
       un[0] += (0.0 + 0.0) * dt;
-      un[1] += mulx<12>(fx1 + fy1, dt);
-      un[2] += mulx<12>(fx2 + fy2, dt);
-      un[3] += mulx<12>(fx3 + fy3, dt);
+      double d1, d2;
+      mulx2<12, SOFT>(fx1 + fy1, dt, fx2 + fy2, dt, d1, d2);
+      un[1] += d1;
+      un[2] += d2;
+      un[3] += mulx<12, SOFT>(fx3 + fy3, dt);
     }
     // RK2 corrector: 0.5 * (U0 + Unew) (Update.h:214-220)
     if (a.stage == STAGE_RK2_CORRECT) {
@@ -513,13 +549,13 @@ __global__ void __launch_bounds__(NT, step_ctas_per_sm<RECON, RS>(VISC))
     for (int k = 0; k < 4; ++k) Udst[k * PL + g] = un[k];
 
     // consToPrim (+ checkNegatives on the final stage)
-    S4<double> q = cons_to_prim(S4<double>{un[0], un[1], un[2], un[3]}, gas);
+    S4<double> q = cons_to_prim<SOFT>(S4<double>{un[0], un[1], un[2], un[3]}, gas);
     if (final_stage) {
       if (fv_lt0(q.r)) { q.r = a.eps_reset; ++cnt_rho; }
       if (fv_lt0(q.p)) { q.p = a.eps_reset; ++cnt_prs; }
       cnt_nan += (unsigned)fv_isnan(q.r) + (unsigned)fv_isnan(q.u) + (unsigned)fv_isnan(q.v) + (unsigned)fv_isnan(q.p);
       // inverse hyperbolic dt of the new state (ComputeDt.h:31-34)
-      const double cs = sound_speed(q, gas);
+      const double cs = sound_speed<SOFT>(q, gas);
       const double ih = ddivc(cs + fabs(q.u), a.dx, a.inv_dx, a.dx_pow2, a.rw_dx) +
                         ddivc(cs + fabs(q.v), a.dy, a.inv_dy, a.dy_pow2, a.rw_dy);
       lmax = fv_fmax(lmax, ih);
@@ -538,19 +574,19 @@ __global__ void __launch_bounds__(NT, step_ctas_per_sm<RECON, RS>(VISC))
     const bool ex = (i < 2 || i >= a.Nx - 2), ey = (j < 2 || j >= a.Ny - 2);
     if (ex || ey) {
       int tx[5], ty[5];
-      bool nx[5], ny[5];
-      tx[0] = i; nx[0] = false;
-      ty[0] = j; ny[0] = false;
-      const int cx = 1 + (ex ? ghost_targets(i, a.Nx, a.bcx, tx + 1, nx + 1) : 0);
-      const int cy = 1 + (ey ? ghost_targets(j, a.Ny, a.bcy, ty + 1, ny + 1) : 0);
+      bool fx[5], fy[5];
+      tx[0] = i; fx[0] = false;
+      ty[0] = j; fy[0] = false;
+      const int cx = 1 + (ex ? ghost_targets(i, a.Nx, a.bcx, tx + 1, fx + 1) : 0);
+      const int cy = 1 + (ey ? ghost_targets(j, a.Ny, a.bcy, ty + 1, fy + 1) : 0);
       for (int b = 0; b < cy; ++b)
         for (int c = 0; c < cx; ++c) {
           if (b == 0 && c == 0) continue;
           const long long gg = (long long)(ty[b] + HALO) * P + (tx[c] + HALO);
           if (!gok(gg, PL)) continue;
           Qd[gg] = q.r;
-          Qd[PL + gg] = nx[c] ? q.u * -1.0 : q.u;
-          Qd[2 * PL + gg] = ny[b] ? q.v * -1.0 : q.v;
+          Qd[PL + gg] = fx[c] ? q.u * -1.0 : q.u;
+          Qd[2 * PL + gg] = fy[b] ? q.v * -1.0 : q.v;
           Qd[3 * PL + gg] = q.p;
         }
     }
