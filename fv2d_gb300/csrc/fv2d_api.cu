@@ -131,6 +131,9 @@ __device__ __forceinline__ double ddiv_c(double x, double d, double inv_d, int p
 __global__ void __launch_bounds__(256) prepare_kernel(PrepArgs a) {
   __shared__ double red[8];
   __shared__ int s_last;
+  __shared__ unsigned long long s_acc;  // largest inverse dt so far (bits)
+  if (threadIdx.x == 0) s_acc = 0ull;
+  __syncthreads();
   const long long n_int = (long long)a.Nx * a.Ny;
   const int W = a.Nx + 4;
   const long long n_ghost = 4LL * W + 4LL * a.Ny;
@@ -155,10 +158,14 @@ __global__ void __launch_bounds__(256) prepare_kernel(PrepArgs a) {
     a.U[a.plane + g] = u.u;
     a.U[2 * a.plane + g] = u.v;
     a.U[3 * a.plane + g] = u.p;
-    const double cs = sound_speed(q, gas);
-    const double ih = ddiv_c(cs + fabs(q.u), a.dx, a.inv_dx, a.dx_pow2, a.rw_dx) +
-                      ddiv_c(cs + fabs(q.v), a.dy, a.inv_dy, a.dy_pow2, a.rw_dy);
-    lmax = fmax(lmax, ih);
+    // where it can exceed the maximum the CTA has reached so far
+    if (may_exceed(inv_dt_bound(q, a.bound), *((volatile unsigned long long *)&s_acc))) {
+      const double cs = sound_speed(q, gas);
+      const double ih = ddiv_c(cs + fabs(q.u), a.dx, a.inv_dx, a.dx_pow2, a.rw_dx) +
+                        ddiv_c(cs + fabs(q.v), a.dy, a.inv_dy, a.dy_pow2, a.rw_dy);
+      if (ih >= 0.0) atomicMax(&s_acc, (unsigned long long)__double_as_longlong(ih));
+      lmax = fmax(lmax, ih);
+    }
   } else if (idx < n_int + n_ghost) {
     long long k = idx - n_int;
     int px, py;  // padded coordinates of the ghost cell
@@ -317,6 +324,7 @@ void fill_args(fv2d_ctx *c) {
   a.CFL = p.CFL;
   a.inv_tc = c->inv_tc;
   a.inv_visc = c->inv_visc;
+  a.bound = dt_bound_of(a.gamma, a.dx, a.dy);
   a.mu = p.mu;
   a.bctc_ymin_value = p.bctc_ymin_value;
   a.bctc_ymax_value = p.bctc_ymax_value;
@@ -397,6 +405,7 @@ int run_prepare(fv2d_ctx *ctx, const double *src) {
   pa.rw_dx = ctx->args.rw_dx;
   pa.rw_dy = ctx->args.rw_dy;
   pa.CFL = p.CFL;
+  pa.bound = ctx->args.bound;
   pa.inv_tc = ctx->inv_tc;
   pa.inv_visc = ctx->inv_visc;
   pa.bcx = p.boundary_x;

@@ -15,9 +15,11 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdint.h>
 
 #include "softfp.cuh"
+#include "step_common.cuh"
 
 namespace fv2d {
 
@@ -254,6 +256,44 @@ __device__ __forceinline__ R sound_speed(const S4<R> &q, const Gas<R> &g) {
 template <int SOFT = kSoftMul, class R>
 __device__ __forceinline__ R sound_speed_r(const S4<R> &q, const Gas<R> &g, uint32_t rr) {
   return dsqrt(fv_div_by(mulx<1, SOFT>(q.p, g.gamma), q.r, rr));
+}
+
+// ---------------------------------------------------------------- CFL filter
+// The CFL reduction needs the largest inverse hyperbolic dt of a grid
+// exactly, so a cell's value only matters when it can exceed a maximum already
+// reached.  inv_dt_bound gives an upper bound of a cell's value in binary32
+// (30-40 instructions and no binary64 ones, against ~350 and 3 for the exact
+// value): the fields truncated to binary32 (relative error below 2^-23 each),
+// the approximate reciprocal and square root (2^-22), half a dozen roundings,
+// all of one sign, within a factor 1 + 2^-18.  States the bound does not cover
+// (negative, infinite, NaN, outside binary32's range) give a NaN, which no
+// test passes over.
+__device__ __forceinline__ float truncated_f32(double x) {  // |x|; 0 below 2^-126, NaN from 2^127 up
+  const uint64_t b = softfp::bits(x);
+  const uint32_t h = (uint32_t)(b >> 32) & 0x7FFFFFFFu;
+  const uint32_t f = h < 0x38100000u ? 0u : ((h - 0x38000000u) << 3) | ((uint32_t)b >> 29);
+  return __uint_as_float(h >= 0x47E00000u ? 0x7FC00000u : f);
+}
+__device__ __forceinline__ float inv_dt_bound(const S4<double> &q, const DtBound &d) {
+  float rr, cs;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rr) : "f"(truncated_f32(q.r)));
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(cs) : "f"(__fmul_rn(__fmul_rn(truncated_f32(q.p), d.gamma), rr)));
+  const float b = __fmul_rn(__fadd_rn(__fmul_rn(__fadd_rn(cs, truncated_f32(q.u)), d.inv_dx),
+                                      __fmul_rn(__fadd_rn(cs, truncated_f32(q.v)), d.inv_dy)),
+                            1.0f + 0x1p-18f);
+  const bool negative = (int32_t)((softfp::bits(q.r) | softfp::bits(q.p)) >> 32) < 0;
+  // a vanishing sound speed may have lost a factor to underflow
+  return negative || !(cs > 0x1p-40f) || !(cs < 0x1p40f) ? __uint_as_float(0x7FC00000u) : b;
+}
+// whether a cell with that bound can exceed the maximum reached so far (the
+// bits of a non-negative double)
+__device__ __forceinline__ bool may_exceed(float bound, uint64_t max_bits) {
+  return !(bound < truncated_f32(softfp::from_bits(max_bits)));
+}
+inline DtBound dt_bound_of(double gamma, double dx, double dy) {
+  const double lo = 1e-30, hi = 1e30;
+  const bool ok = dx > lo && dx < hi && dy > lo && dy < hi && gamma > 1e-6 && gamma < 1e6;
+  return ok ? DtBound{(float)gamma, (float)(1.0 / dx), (float)(1.0 / dy)} : DtBound{NAN, NAN, NAN};
 }
 
 // Update.h:77-85

@@ -52,6 +52,11 @@ struct DevState {
   int pad;
 };
 
+// Constants of the binary32 bound on a cell's inverse dt (physics.cuh).
+struct DtBound {
+  float gamma, inv_dx, inv_dy;  // NaN: no bound, every cell is evaluated
+};
+
 // Everything one step launch needs besides the two tensor maps.
 struct StepArgs {
   double *Q[2];       // primitive planes (4 planes, ghosts included)
@@ -78,6 +83,7 @@ struct StepArgs {
   double gxf, gyf;      // constant gravity narrowed to float (Gravity.h:39)
   double eps_reset;     // epsilon_reset_negative
   double CFL, inv_tc, inv_visc;  // dt finalisation (ComputeDt.h:64)
+  DtBound bound;  // binary32 bound of a cell's inverse dt
   double mu;
   double bctc_ymin_value, bctc_ymax_value;
   int bcx, bcy;
@@ -100,6 +106,7 @@ struct PrepArgs {
   int dx_pow2, dy_pow2;
   uint32_t rw_dx, rw_dy;
   double CFL, inv_tc, inv_visc;
+  DtBound bound;
   int bcx, bcy;
 };
 

@@ -417,6 +417,8 @@ __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
   double *Qd = a.Q[dst];
   const long long PL = a.plane;
   const int P = a.pitch;
+  // the dt reduction as other CTAs have left it (any value it has had will do)
+  const uint64_t acc = *((volatile unsigned long long *)&st->acc_hyp);
 
 #pragma unroll 1
   for (int cidx = tid; cidx < TX * TY; cidx += NT) {
@@ -554,11 +556,14 @@ __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
       if (fv_lt0(q.r)) { q.r = a.eps_reset; ++cnt_rho; }
       if (fv_lt0(q.p)) { q.p = a.eps_reset; ++cnt_prs; }
       cnt_nan += (unsigned)fv_isnan(q.r) + (unsigned)fv_isnan(q.u) + (unsigned)fv_isnan(q.v) + (unsigned)fv_isnan(q.p);
-      // inverse hyperbolic dt of the new state (ComputeDt.h:31-34)
-      const double cs = sound_speed<SOFT>(q, gas);
-      const double ih = ddivc(cs + fabs(q.u), a.dx, a.inv_dx, a.dx_pow2, a.rw_dx) +
-                        ddivc(cs + fabs(q.v), a.dy, a.inv_dy, a.dy_pow2, a.rw_dy);
-      lmax = fv_fmax(lmax, ih);
+      // inverse hyperbolic dt of the new state (ComputeDt.h:31-34), where it
+      // can exceed what other CTAs have already reached
+      if (may_exceed(inv_dt_bound(q, a.bound), acc)) {
+        const double cs = sound_speed<SOFT>(q, gas);
+        const double ih = ddivc(cs + fabs(q.u), a.dx, a.inv_dx, a.dx_pow2, a.rw_dx) +
+                          ddivc(cs + fabs(q.v), a.dy, a.inv_dy, a.dy_pow2, a.rw_dy);
+        lmax = fv_fmax(lmax, ih);
+      }
     }
     Qd[g] = q.r;
     Qd[PL + g] = q.u;
