@@ -70,4 +70,26 @@ inline int choose_band(const std::vector<BandGrid> &grids, double resident_warps
   return kMinBand;
 }
 
+// Band height of a march lane that can run in one wave: the shortest that gives
+// it no more items than the resident warps, or 0 when that takes bands taller
+// than kMaxWaveBand (choose_band then picks).  A lane with fewer items than warps
+// is bound by the chain of a work item's rows (1.4 us a row, 4 rows of window
+// fill beside the band's), not by throughput, so shorter bands shorten the step
+// until the warps are used up; and at 8 to 12 rows one full wave beats the next
+// shorter band's wave and a bit.  Measured, ms per 100 steps, choose_band | this:
+// KH 128^2 2.03 | 1.11, 256^2 2.07 | 1.06, 512^2 2.20 | 1.52; RT 128 x 384
+// 1.77 | 1.23, 512 x 1536 3.46 | 3.09 (10 rows).  Several such lanes side by side
+// do best with every lane sized as if alone (16 mixed grids: 5.63 against 6.08
+// with the warps shared out).  Where a full wave needs taller bands the plentiful
+// items of choose_band are as good (KH 2048^2: 30 rows 17.4, 12 rows 18.0).
+constexpr int kMaxWaveBand = 12;
+inline int choose_wave_band(const std::vector<BandGrid> &grids, double warps) {
+  for (int H = 1; H <= kMaxWaveBand; ++H) {
+    double items = 0;
+    for (const BandGrid &g : grids) items += (double)g.strips * ((g.Ny + H - 1) / H);
+    if (items <= warps) return H;
+  }
+  return 0;
+}
+
 }  // namespace fv2d

@@ -402,6 +402,13 @@ size_t state_bytes(const fv2d_params &p, int *pitch, long long *plane, size_t *r
   return needs_rows(p) ? *rows_off + sizeof(float) * kRowStride * (size_t)p.Ny : planes;
 }
 
+// Resident warps of a configuration's launch.
+double lane_warps(const fv2d_server *s, int cfg) {
+  int nt;
+  batch_cfg_info(cfg, nullptr, nullptr, &nt, nullptr, nullptr, nullptr, nullptr);
+  return (double)s->cfg_grid[cfg] * (nt / 32);
+}
+
 int lane_cfg(const fv2d_server *s, int lane) { return s->fam_cfg[lane / kBuckets][lane % kBuckets]; }
 
 // Lane of a request: its grid-size bucket + kBuckets * its family; with
@@ -457,7 +464,8 @@ int admit(fv2d_server *s, const Pending &pd) {
   int tx, ty, nt, staging;
   batch_cfg_info(cfg, &tx, &ty, &nt, &staging, nullptr, nullptr, nullptr);
   // the march kernels' band height changes with the lane's contents: room for
-  // the most items it can take
+  // the most items it can take (bands below kMinBand only while they fit the
+  // resident warps)
   const int items = ((Nx + tx - 1) / tx) * ((Ny + (staging == 2 ? kMinBand : ty) - 1) / (staging == 2 ? kMinBand : ty));
   float bg_r = 0.f, bg_e = 0.f;
   if (pd.id > 0) background(r, &bg_r, &bg_e);  // the autotuner's synthetic states need none
@@ -465,7 +473,7 @@ int admit(fv2d_server *s, const Pending &pd) {
   // lists (that synchronises the stream and drops the captured graphs)
   void *mem = s->arena.alloc(bytes);
   if (!mem) return -1;
-  if (!reserve_work(s, lane, s->items_in[lane] + items)) {
+  if (!reserve_work(s, lane, std::max(s->items_in[lane] + items, (int)lane_warps(s, cfg)))) {
     s->arena.release(mem, bytes);
     return -1;
   }
@@ -649,7 +657,9 @@ int lane_band(const fv2d_server *s, int lane, const std::vector<int> &slots) {
   std::vector<BandGrid> grids;
   grids.reserve(slots.size());
   for (int k : slots) grids.push_back(BandGrid{s->h_up[k].ntx, s->h_up[k].Ny});
-  return choose_band(grids, (double)s->cfg_grid[c] * (nt / 32));
+  const double warps = lane_warps(s, c);
+  if (const int H = choose_wave_band(grids, warps)) return H;
+  return choose_band(grids, warps);
 }
 
 void rebuild_lists(fv2d_server *s) {
