@@ -583,6 +583,7 @@ int fv2d_create(const fv2d_params *p, int device, fv2d_ctx **out) {
   std::memset(&s0, 0, sizeof(s0));
   s0.status = RUN_PAUSED;
   s0.log_cap = ctx->log_cap;
+  s0.one = 1.0;
   if ((e = cudaMemcpy(ctx->st, &s0, sizeof(s0), cudaMemcpyHostToDevice)) != cudaSuccess)
     return bail(cuda_fail(ctx, e, "cudaMemcpy state"));
   if (int rc = encode_maps(ctx)) return bail(rc);

@@ -117,41 +117,72 @@ __host__ __device__ __forceinline__ float fv_mul(float x, float y) { return x * 
 __host__ __device__ __forceinline__ bool fv_isnan(float x) { return isnan(x); }
 
 // Products moved from the binary64 pipe to the integer pipes (softfp::mul_rn),
-// by group: a product holds the binary64 pipe for 64 cycles of an SM
-// sub-partition, an integer-pipe one the ALU for about as long, so the set
-// that balances the two is the fastest.  The set is a mask (bit
-// GROUP - 1 set: that group on the integer pipes); the groups are
-//   1  HLLC: squared velocities, p gamma, u* numerator, fluxes
+// by group: a product holds the binary64 pipe for 76 cycles of an SM
+// sub-partition, an integer-pipe one the ALU for about 80, so the set that
+// balances the two is the fastest.  The sets are masks (bit GROUP - 1: that
+// group on the integer pipes); the groups are
+//   1  HLLC: squared velocities
 //   2  HLLC: total energy (rho/2 (u^2 + v^2), p / (gamma - 1))
 //   3  the update's dt (F_L - F_R) products
 //   4  consToPrim: kinetic energy and (E - Ek)(gamma - 1)
 //   5  HLLC: rho (u - S)
 //   6  HLLC: p* numerator
 //   7  HLLC: star energy
-//   8  (unused)
+//   8  HLLC: fluxes
 //   9  HLL: products of each side's state (kinetic energy, fluxes, momenta)
 //  10  HLL: the HLL average's products by the wave speeds
 //  11  viscous face terms
 //  12  conduction fluxes and the conduction / viscosity update products
 //  13  MUSCL-Hancock predictor
 //  14  FSLP
-// Measured (ms per step; group on the binary64 pipe | on the integer pipes):
-// KH 2048^2 HLLC: 5 and 6 1.10 | 1.12, 7 1.10 | 1.13; Sedov 2048^2: 2 1.01 |
-// 0.99; FSLP RK2 777 x 1501: 14 0.372 | 0.358; RT 1024 x 3072: 12 1.68 | 1.64.
-// The viscous kernels also move group 10 (1.64 | 1.60); without viscosity it
-// is slower there (PCM-HLL 1000 x 600: 1.53 | 1.63 for five steps).
-#ifndef FV2D_SOFT_MUL
-#define FV2D_SOFT_MUL 14607
+//  15  HLLC: u* numerator
+// Measured (ms a step; group on the binary64 pipe | on the integer pipes):
+// Sedov 2048^2 HLLC: 1 0.96 | 0.94, 3 1.00 | 0.94, 8 1.00 | 0.96; KH 2048^2
+// HLLC: 4 1.02 | 1.07, 6 1.02 | 1.06, 7 1.05 | 1.06; its PCM form: 5 0.80 | 0.77;
+// HLL: 9 1.58 | 1.40; FSLP RK2 777 x 1501: 3 0.327 | 0.334 a stage; RT
+// 1024 x 3072: 10 1.64 | 1.60, 12 1.48 | 1.46.
+constexpr int kSoftMulHllc = 31127, kSoftMul = kSoftMulHllc & ~4, kSoftMulVisc = kSoftMul | 512;
+// Sums and differences.  In binary64 on the device a + b is issued as the
+// multiply-add a * one + b, with `one` = 1 in a register that the compiler
+// cannot see through: the same correctly rounded sum (signed zeros, infinities
+// and NaNs included), but GB300 takes a warp's three-register DFMA every 64
+// cycles of an SM sub-partition and a DADD or DMUL (or a DFMA with a constant
+// operand) only every 76 (measured: 100 % against 84 % of the pipe's peak), and
+// the step is bound by that pipe: KH 2048^2 1.08 -> 1.02 ms a step, Sedov 0.99 ->
+// 0.94, RT 1024 x 3072 1.54 -> 1.48.  Products stay DMULs: a register pair for
+// their -0 addend cost as much as it gave.
+template <class R>
+struct Adder {
+  R one = R(1);
+  __host__ __device__ __forceinline__ R operator()(R a, R b) const { return a + b; }
+  __host__ __device__ __forceinline__ R sub(R a, R b) const { return a - b; }
+};
+template <>
+struct Adder<double> {
+  double one = 1.0;
+  __host__ __device__ __forceinline__ double operator()(double a, double b) const {
+#ifdef __CUDA_ARCH__
+    return __fma_rn(a, one, b);
+#else
+    return a + b;
 #endif
-constexpr int kSoftMul = FV2D_SOFT_MUL, kSoftMulVisc = FV2D_SOFT_MUL | 512;
-template <int GROUP, int SOFT = kSoftMul, class R>
+  }
+  __host__ __device__ __forceinline__ double sub(double a, double b) const {
+#ifdef __CUDA_ARCH__
+    return __fma_rn(-b, one, a);
+#else
+    return a - b;
+#endif
+  }
+};
+
+template <int GROUP, int SOFT, class R>
 __host__ __device__ __forceinline__ R mulx(R a, R b) {
   if constexpr ((SOFT >> (GROUP - 1)) & 1) return fv_mul(a, b);
   else return a * b;
 }
-
 // {x0 y0, x1 y1} of one group: on the integer pipes in one call
-template <int GROUP, int SOFT = kSoftMul, class R>
+template <int GROUP, int SOFT, class R>
 __host__ __device__ __forceinline__ void mulx2(R x0, R y0, R x1, R y1, R &r0, R &r1) {
 #ifdef __CUDA_ARCH__
   if constexpr (sizeof(R) == 8 && ((SOFT >> (GROUP - 1)) & 1)) {
@@ -210,11 +241,12 @@ struct Gas {
   R entho;   // 1.0 / (gamma0 - 1.0)               (RiemannSolvers.h:76)
   R fslp_K;  // FSLP K                              (SimInfo.h:399)
   uint32_t rgm1;  // fv_recip(gm1): the divisions by gamma0 - 1 (set by make_gas)
+  Adder<R> add;
 };
 
 template <class R>
-__host__ __device__ __forceinline__ Gas<R> make_gas(R gamma, R gm1, R entho, R fslp_K) {
-  return Gas<R>{gamma, gm1, entho, fslp_K, fv_recip(gm1)};
+__host__ __device__ __forceinline__ Gas<R> make_gas(R gamma, R gm1, R entho, R fslp_K, Adder<R> add = Adder<R>()) {
+  return Gas<R>{gamma, gm1, entho, fslp_K, fv_recip(gm1), add};
 }
 
 // States.h:19-30
@@ -237,8 +269,8 @@ __host__ __device__ __forceinline__ S4<R> cons_to_prim(const S4<R> &u, const Gas
   fv_div2(u.u, u.v, u.r, q.u, q.v);
   R uu, vv;
   mulx2<4, SOFT>(q.u, q.u, q.v, q.v, uu, vv);
-  R Ek = mulx<4, SOFT>(fv_half(q.r), uu + vv);
-  q.p = mulx<4, SOFT>(u.p - Ek, g.gm1);
+  R Ek = mulx<4, SOFT>(fv_half(q.r), g.add(uu, vv));
+  q.p = mulx<4, SOFT>(g.add.sub(u.p, Ek), g.gm1);
   return q;
 }
 
@@ -326,25 +358,25 @@ __device__ __forceinline__ void riemann_hll(const S4<R> &qL, const S4<R> &qR, S4
   // term of primToCons below: the same division, evaluated once.
   const R peL = fv_div_by(qL.p, g.gm1, g.rgm1);
   const R peR = fv_div_by(qR.p, g.gm1, g.rgm1);
-  const R EkL = mulx<9>(fv_half(qL.r), mulx<9>(qL.u, qL.u) + mulx<9>(qL.v, qL.v));
-  const R EkR = mulx<9>(fv_half(qR.r), mulx<9>(qR.u, qR.u) + mulx<9>(qR.v, qR.v));
+  const R EkL = (fv_half(qL.r) * ((qL.u * qL.u) + (qL.v * qL.v)));
+  const R EkR = (fv_half(qR.r) * ((qR.u * qR.u) + (qR.v * qR.v)));
   const R EL = (peL + EkL);
   const R ER = (peR + EkR);
-  const R ruL = mulx<9>(qL.r, qL.u), ruR = mulx<9>(qR.r, qR.u);
-  S4<R> FL{ruL, mulx<9>(ruL, qL.u) + qL.p, mulx<9>(ruL, qL.v), mulx<9>(qL.p + EL, qL.u)};
-  S4<R> FR{ruR, mulx<9>(ruR, qR.u) + qR.p, mulx<9>(ruR, qR.v), mulx<9>(qR.p + ER, qR.u)};
+  const R ruL = (qL.r * qL.u), ruR = (qR.r * qR.u);
+  S4<R> FL{ruL, (ruL * qL.u) + qL.p, (ruL * qL.v), ((qL.p + EL) * qL.u)};
+  S4<R> FR{ruR, (ruR * qR.u) + qR.p, (ruR * qR.v), ((qR.p + ER) * qR.u)};
   // primToCons (States.h:19-30) of both states
-  const R mvL = mulx<9>(qL.r, qL.v), mvR = mulx<9>(qR.r, qR.v);
-  const R uEL = (fv_div_by(fv_half(mulx<9>(ruL, ruL) + mulx<9>(mvL, mvL)), qL.r, rL) + peL);
-  const R uER = (fv_div_by(fv_half(mulx<9>(ruR, ruR) + mulx<9>(mvR, mvR)), qR.r, rR) + peR);
-  const R SLSR = mulx<10>(SL, SR);
+  const R mvL = (qL.r * qL.v), mvR = (qR.r * qR.v);
+  const R uEL = (fv_div_by(fv_half((ruL * ruL) + (mvL * mvL)), qL.r, rL) + peL);
+  const R uER = (fv_div_by(fv_half((ruR * ruR) + (mvR * mvR)), qR.r, rR) + peR);
+  const R SLSR = (SL * SR);
   const R den = SR - SL;
   const uint32_t rden = fv_recip(den);
   S4<R> FM;
-  FM.r = fv_div_by(mulx<10>(SR, FL.r) - mulx<10>(SL, FR.r) + mulx<10>(SLSR, qR.r - qL.r), den, rden);
-  FM.u = fv_div_by(mulx<10>(SR, FL.u) - mulx<10>(SL, FR.u) + mulx<10>(SLSR, ruR - ruL), den, rden);
-  FM.v = fv_div_by(mulx<10>(SR, FL.v) - mulx<10>(SL, FR.v) + mulx<10>(SLSR, mvR - mvL), den, rden);
-  FM.p = fv_div_by(mulx<10>(SR, FL.p) - mulx<10>(SL, FR.p) + mulx<10>(SLSR, uER - uEL), den, rden);
+  FM.r = fv_div_by((SR * FL.r) - (SL * FR.r) + (SLSR * (qR.r - qL.r)), den, rden);
+  FM.u = fv_div_by((SR * FL.u) - (SL * FR.u) + (SLSR * (ruR - ruL)), den, rden);
+  FM.v = fv_div_by((SR * FL.v) - (SL * FR.v) + (SLSR * (mvR - mvL)), den, rden);
+  FM.p = fv_div_by((SR * FL.p) - (SL * FR.p) + (SLSR * (uER - uEL)), den, rden);
   const R pM = fv_half(qL.p + qR.p);
   const bool left = fv_ge0(SL);
   const bool right = !left && fv_le0(SR);
@@ -361,41 +393,42 @@ template <int SOFT = kSoftMul>
 __device__ __forceinline__ void riemann_hll(const S4<double> &qL, const S4<double> &qR, S4<double> &f, double &pout,
                                             const Gas<double> &g) {
   const double2 c = softfp::sound2(qL.p, qL.r, qR.p, qR.r, g.gamma);
-  const double SL = fv_fmin(qL.u - c.x, qR.u - c.y);
-  const double SR = fv_fmax(qL.u + c.x, qR.u + c.y);
+  const Adder<double> add = g.add;
+  const double SL = fv_fmin(add.sub(qL.u, c.x), add.sub(qR.u, c.y));
+  const double SR = fv_fmax(add(qL.u, c.x), add(qR.u, c.y));
   double peL, peR, uuL, vvL, uuR, vvR, EkL, EkR, EL, ER;
   fv_div2_by(qL.p, qR.p, g.gm1, g.rgm1, peL, peR);
   mulx2<9, SOFT>(qL.u, qL.u, qL.v, qL.v, uuL, vvL);
   mulx2<9, SOFT>(qR.u, qR.u, qR.v, qR.v, uuR, vvR);
-  mulx2<9, SOFT>(fv_half(qL.r), uuL + vvL, fv_half(qR.r), uuR + vvR, EkL, EkR);
-  EL = peL + EkL;
-  ER = peR + EkR;
+  mulx2<9, SOFT>(fv_half(qL.r), add(uuL, vvL), fv_half(qR.r), add(uuR, vvR), EkL, EkR);
+  EL = add(peL, EkL);
+  ER = add(peR, EkR);
   S4<double> FL, FR;
   double a, b, mvL, mvR;
   mulx2<9, SOFT>(qL.r, qL.u, qR.r, qR.u, FL.r, FR.r);
   mulx2<9, SOFT>(FL.r, qL.u, FR.r, qR.u, a, b);
-  FL.u = a + qL.p;
-  FR.u = b + qR.p;
+  FL.u = add(a, qL.p);
+  FR.u = add(b, qR.p);
   mulx2<9, SOFT>(FL.r, qL.v, FR.r, qR.v, FL.v, FR.v);
-  mulx2<9, SOFT>(qL.p + EL, qL.u, qR.p + ER, qR.u, FL.p, FR.p);
+  mulx2<9, SOFT>(add(qL.p, EL), qL.u, add(qR.p, ER), qR.u, FL.p, FR.p);
   mulx2<9, SOFT>(qL.r, qL.v, qR.r, qR.v, mvL, mvR);
   mulx2<9, SOFT>(FL.r, FL.r, mvL, mvL, uuL, vvL);
   mulx2<9, SOFT>(FR.r, FR.r, mvR, mvR, uuR, vvR);
   double wL, wR;
-  fv_quot2(fv_half(uuL + vvL), qL.r, fv_half(uuR + vvR), qR.r, wL, wR);
-  const double duE = (wR + peR) - (wL + peL);
+  fv_quot2(fv_half(add(uuL, vvL)), qL.r, fv_half(add(uuR, vvR)), qR.r, wL, wR);
+  const double duE = add.sub(add(wR, peR), add(wL, peL));
   const double SLSR = mulx<10, SOFT>(SL, SR);
-  const double den = SR - SL;
+  const double den = add.sub(SR, SL);
   const uint32_t rden = fv_recip(den);
   auto average = [&](double fL, double fR, double du) {
     double x, y;
     mulx2<10, SOFT>(SR, fL, SL, fR, x, y);
-    return x - y + mulx<10, SOFT>(SLSR, du);
+    return add(add.sub(x, y), mulx<10, SOFT>(SLSR, du));
   };
   S4<double> FM;
-  fv_div2_by(average(FL.r, FR.r, qR.r - qL.r), average(FL.u, FR.u, FR.r - FL.r), den, rden, FM.r, FM.u);
-  fv_div2_by(average(FL.v, FR.v, mvR - mvL), average(FL.p, FR.p, duE), den, rden, FM.v, FM.p);
-  const double pM = fv_half(qL.p + qR.p);
+  fv_div2_by(average(FL.r, FR.r, add.sub(qR.r, qL.r)), average(FL.u, FR.u, add.sub(FR.r, FL.r)), den, rden, FM.r, FM.u);
+  fv_div2_by(average(FL.v, FR.v, add.sub(mvR, mvL)), average(FL.p, FR.p, duE), den, rden, FM.v, FM.p);
+  const double pM = fv_half(add(qL.p, qR.p));
   const bool left = fv_ge0(SL);
   const bool right = !left && fv_le0(SR);
   f.r = left ? FL.r : (right ? FR.r : FM.r);
@@ -412,20 +445,20 @@ template <class R>
 __device__ __forceinline__ void riemann_hllc(const S4<R> &qL, const S4<R> &qR, S4<R> &f, R &pout, const Gas<R> &g) {
   const R rL = qL.r, uL = qL.u, vL = qL.v, pL = qL.p;
   const R rR = qR.r, uR = qR.u, vR = qR.v, pR = qR.p;
-  const R ekL = mulx<2>(fv_half(rL), mulx<1>(uL, uL) + mulx<1>(vL, vL));
-  const R EL = ekL + mulx<1>(pL, g.entho);
-  const R ekR = mulx<2>(fv_half(rR), mulx<1>(uR, uR) + mulx<1>(vR, vR));
-  const R ER = ekR + mulx<1>(pR, g.entho);
+  const R ekL = (fv_half(rL) * ((uL * uL) + (vL * vL)));
+  const R EL = ekL + (pL * g.entho);
+  const R ekR = (fv_half(rR) * ((uR * uR) + (vR * vR)));
+  const R ER = ekR + (pR * g.entho);
   const R cL = sound_speed(qL, g);
   const R cR = sound_speed(qR, g);
   const R cmax = fv_fmax(cL, cR);
   const R SL = fv_fmin(uL, uR) - cmax;
   const R SR = fv_fmax(uL, uR) + cmax;
-  const R rcL = mulx<5>(rL, uL - SL);
-  const R rcR = mulx<5>(rR, SR - uR);
+  const R rcL = (rL * (uL - SL));
+  const R rcR = (rR * (SR - uR));
   R uS, pS;
-  fv_div2(mulx<1>(rcR, uR) + mulx<1>(rcL, uL) + (pL - pR),
-          mulx<6>(rcR, pL) + mulx<6>(rcL, pR) + mulx<6>(mulx<6>(rcL, rcR), uL - uR), rcR + rcL, uS, pS);
+  fv_div2((rcR * uR) + (rcL * uL) + (pL - pR),
+          (rcR * pL) + (rcL * pR) + ((rcL * rcR) * (uL - uR)), rcR + rcL, uS, pS);
   const bool sideL = fv_gt0(uS);
   const R rK = sideL ? rL : rR;
   const R uK = sideL ? uL : uR;
@@ -433,7 +466,7 @@ __device__ __forceinline__ void riemann_hllc(const S4<R> &qL, const S4<R> &qR, S
   const R EK = sideL ? EL : ER;
   const R SK = sideL ? SL : SR;
   R rS, ES;
-  fv_div2(mulx<7>(rK, SK - uK), mulx<7>(SK - uK, EK) - mulx<7>(pK, uK) + mulx<7>(pS, uS), SK - uS, rS, ES);
+  fv_div2((rK * (SK - uK)), ((SK - uK) * EK) - (pK * uK) + (pS * uS), SK - uS, rS, ES);
   // branch order of RiemannSolvers.h:89-112
   const bool bL = fv_gt0(SL);
   const bool bStar = !bL && (sideL || fv_gt0(SR));
@@ -446,10 +479,10 @@ __device__ __forceinline__ void riemann_hllc(const S4<R> &qL, const S4<R> &qR, S
     sr = rR; su = uR; sv = vR; sp = pR; E = ER;
   }
   pout = sp;
-  f.r = mulx<1>(sr, su);
-  f.u = mulx<1>(mulx<1>(sr, su), su) + sp;
-  f.v = mulx<1>(f.r, sv);
-  f.p = mulx<8>(E + sp, su);
+  f.r = (sr * su);
+  f.u = ((sr * su) * su) + sp;
+  f.v = (f.r * sv);
+  f.p = ((E + sp) * su);
 }
 
 // x with its sign changed, a zero as it is: (b - a) from (a - b), whose zero
@@ -473,14 +506,16 @@ __device__ __forceinline__ void riemann_hllc(const S4<double> &qL, const S4<doub
   const double rR = qR.r, uR = qR.u, vR = qR.v, pR = qR.p;
   const double cmax = softfp::sound_max(pL, rL, pR, rR, g.gamma);
   const double2 um = softfp::minmax_nm(uL, uR);
-  const double SL = um.x - cmax, SR = um.y + cmax;
-  const double dL = uL - SL, dR = SR - uR;
+  const Adder<double> add = g.add;
+  const double SL = add.sub(um.x, cmax), SR = add(um.y, cmax);
+  const double dL = add.sub(uL, SL), dR = add.sub(SR, uR);
   double rcL, rcR, a, b, c, d;
   mulx2<5, SOFT>(rL, dL, rR, dR, rcL, rcR);
-  mulx2<1, SOFT>(rcR, uR, rcL, uL, a, b);
+  mulx2<15, SOFT>(rcR, uR, rcL, uL, a, b);
   mulx2<6, SOFT>(rcR, pL, rcL, pR, c, d);
   double uS, pS;
-  fv_div2(a + b + (pL - pR), c + d + mulx<6, SOFT>(mulx<6, SOFT>(rcL, rcR), uL - uR), rcR + rcL, uS, pS);
+  fv_div2(add(add(a, b), add.sub(pL, pR)),
+          add(add(c, d), mulx<6, SOFT>(mulx<6, SOFT>(rcL, rcR), add.sub(uL, uR))), add(rcR, rcL), uS, pS);
   const bool sideL = fv_gt0(uS);
   // branch order of RiemannSolvers.h:89-112
   const bool bL = fv_gt0(SL);
@@ -495,18 +530,18 @@ __device__ __forceinline__ void riemann_hllc(const S4<double> &qL, const S4<doub
   const double rcK = left ? negated_difference(rcL) : rcR;  // rho_K (S_K - u_K)
   double E;
   mulx2<1, SOFT>(su, su, sv, sv, a, b);
-  mulx2<2, SOFT>(fv_half(sr), a + b, sp, g.entho, c, d);
-  E = c + d;
+  mulx2<2, SOFT>(fv_half(sr), add(a, b), sp, g.entho, c, d);
+  E = add(c, d);
   double rS, ES;
   mulx2<7, SOFT>(dK, E, sp, su, a, b);
-  fv_div2(rcK, a - b + mulx<7, SOFT>(pS, uS), SK - uS, rS, ES);
+  fv_div2(rcK, add(add.sub(a, b), mulx<7, SOFT>(pS, uS)), add.sub(SK, uS), rS, ES);
   if (bStar) {
     sr = rS; su = uS; sp = pS; E = ES;
   }
   pout = sp;
-  mulx2<1, SOFT>(sr, su, E + sp, su, f.r, f.p);
-  mulx2<1, SOFT>(f.r, su, f.r, sv, a, f.v);
-  f.u = a + sp;
+  mulx2<8, SOFT>(sr, su, add(E, sp), su, f.r, f.p);
+  mulx2<8, SOFT>(f.r, su, f.r, sv, a, f.v);
+  f.u = add(a, sp);
 }
 
 // RiemannSolvers.h:130-171 (Kokkos::max / min as (a<b)?b:a and (b<a)?b:a).
@@ -514,28 +549,28 @@ template <class R>
 __device__ __forceinline__ void riemann_fslp(const S4<R> &qL, const S4<R> &qR, S4<R> &f, R &pout, R gdx,
                                              const Gas<R> &g) {
   const R rhoL = qL.r, uL = qL.u, pL = qL.p;
-  const R csL = dsqrt(fv_div(mulx<14>(g.gamma, pL), rhoL));
+  const R csL = dsqrt(fv_div((g.gamma * pL), rhoL));
   const R rhoR = qR.r, uR = qR.u, pR = qR.p;
-  const R csR = dsqrt(fv_div(mulx<14>(g.gamma, pR), rhoR));
-  const R zL = mulx<14>(rhoL, csL), zR = mulx<14>(rhoR, csR);
-  const R ai = mulx<14>(g.fslp_K, fv_lt(zL, zR) ? zR : zL);
+  const R csR = dsqrt(fv_div((g.gamma * pR), rhoR));
+  const R zL = (rhoL * csL), zR = (rhoR * csR);
+  const R ai = (g.fslp_K * (fv_lt(zL, zR) ? zR : zL));
   const R mL = fv_div(fabs(uL), csL), mR = fv_div(fabs(uR), csR);
   const R mx = fv_lt(mL, mR) ? mR : mL;
   const R theta = fv_lt(mx, R(1)) ? mx : R(1);
-  const R ustar = fv_half(uR + uL) - mulx<14>(fv_div(R(0.5), ai), pR - pL - mulx<14>(fv_half(rhoL + rhoR), gdx));
-  const R Pi = fv_half(pR + pL) - mulx<14>(mulx<14>(fv_half(theta), ai), uR - uL);
+  const R ustar = fv_half(uR + uL) - ((fv_div(R(0.5), ai)) * (pR - pL - (fv_half(rhoL + rhoR) * gdx)));
+  const R Pi = fv_half(pR + pL) - (((fv_half(theta) * ai)) * (uR - uL));
   const bool up = fv_gt0(ustar);
   const R sr = up ? qL.r : qR.r;
   const R su = up ? qL.u : qR.u;
   const R sv = up ? qL.v : qR.v;
   const R sp = up ? qL.p : qR.p;
-  const R Ekstar = mulx<14>(fv_half(sr), mulx<14>(su, su) + mulx<14>(sv, sv));
+  const R Ekstar = (fv_half(sr) * ((su * su) + (sv * sv)));
   const R Estar = Ekstar + fv_div_by(sp, g.gm1, g.rgm1);
-  const R usr = mulx<14>(ustar, sr);
+  const R usr = (ustar * sr);
   f.r = usr;
-  f.u = mulx<14>(usr, su) + Pi;
-  f.v = mulx<14>(usr, sv);
-  f.p = mulx<14>(ustar, Estar + Pi);
+  f.u = (usr * su) + Pi;
+  f.v = (usr * sv);
+  f.p = (ustar * (Estar + Pi));
   pout = Pi;
 }
 
@@ -545,6 +580,7 @@ __device__ __forceinline__ void riemann_fslp(const S4<double> &qL, const S4<doub
                                              double gdx, const Gas<double> &g) {
   const double uL = qL.u, pL = qL.p, uR = qR.u, pR = qR.p;
   const double2 c = softfp::sound2(pL, qL.r, pR, qR.r, g.gamma);
+  const Adder<double> add = g.add;
   double zL, zR, mL, mR;
   mulx2<14, SOFT>(qL.r, c.x, qR.r, c.y, zL, zR);
   const double ai = mulx<14, SOFT>(g.fslp_K, fv_lt(zL, zR) ? zR : zL);
@@ -552,22 +588,22 @@ __device__ __forceinline__ void riemann_fslp(const S4<double> &qL, const S4<doub
   const double mx = fv_lt(mL, mR) ? mR : mL;
   const double theta = fv_lt(mx, 1.0) ? mx : 1.0;
   double a, b, uu, vv, w, z;
-  mulx2<14, SOFT>(fv_half(qL.r + qR.r), gdx, fv_half(theta), ai, a, b);
-  mulx2<14, SOFT>(fv_div(0.5, ai), pR - pL - a, b, uR - uL, a, b);
-  const double ustar = fv_half(uR + uL) - a;
-  const double Pi = fv_half(pR + pL) - b;
+  mulx2<14, SOFT>(fv_half(add(qL.r, qR.r)), gdx, fv_half(theta), ai, a, b);
+  mulx2<14, SOFT>(fv_div(0.5, ai), add.sub(add.sub(pR, pL), a), b, add.sub(uR, uL), a, b);
+  const double ustar = add.sub(fv_half(add(uR, uL)), a);
+  const double Pi = add.sub(fv_half(add(pR, pL)), b);
   const bool up = fv_gt0(ustar);
   const double sr = up ? qL.r : qR.r;
   const double su = up ? uL : uR;
   const double sv = up ? qL.v : qR.v;
   const double sp = up ? pL : pR;
   mulx2<14, SOFT>(su, su, sv, sv, uu, vv);
-  mulx2<14, SOFT>(fv_half(sr), uu + vv, ustar, sr, w, z);
-  const double Estar = w + fv_div_by(sp, g.gm1, g.rgm1);
+  mulx2<14, SOFT>(fv_half(sr), add(uu, vv), ustar, sr, w, z);
+  const double Estar = add(w, fv_div_by(sp, g.gm1, g.rgm1));
   f.r = z;
   mulx2<14, SOFT>(z, su, z, sv, a, f.v);
-  f.u = a + Pi;
-  f.p = mulx<14, SOFT>(ustar, Estar + Pi);
+  f.u = add(a, Pi);
+  f.p = mulx<14, SOFT>(ustar, add(Estar, Pi));
   pout = Pi;
 }
 
@@ -598,16 +634,29 @@ __device__ __forceinline__ void riemann(const S4<float> &qL, const S4<float> &qR
 // Extension (no reference counterpart): primitive-variable MUSCL-Hancock
 // half-step qh = q - (dt/2dx) A(q) sx - (dt/2dy) B(q) sy, with ax = 0.5 dt/dx,
 // ay = 0.5 dt/dy and sx, sy the full minmod slopes.
-template <int SOFT = kSoftMul, class R>
+template <class R>
 __host__ __device__ __forceinline__ S4<R> hancock(const S4<R> &q, const S4<R> &sx, const S4<R> &sy, R ax, R ay,
                                                   R gamma) {
   S4<R> h;
-  h.r = q.r - (mulx<13, SOFT>(ax, mulx<13, SOFT>(q.u, sx.r) + mulx<13, SOFT>(q.r, sx.u)) +
-               mulx<13, SOFT>(ay, mulx<13, SOFT>(q.v, sy.r) + mulx<13, SOFT>(q.r, sy.v)));
-  h.u = q.u - (mulx<13, SOFT>(ax, mulx<13, SOFT>(q.u, sx.u) + fv_div(sx.p, q.r)) + mulx<13, SOFT>(ay, mulx<13, SOFT>(q.v, sy.u)));
-  h.v = q.v - (mulx<13, SOFT>(ax, mulx<13, SOFT>(q.u, sx.v)) + mulx<13, SOFT>(ay, mulx<13, SOFT>(q.v, sy.v) + fv_div(sy.p, q.r)));
-  h.p = q.p - (mulx<13, SOFT>(ax, mulx<13, SOFT>(mulx<13, SOFT>(gamma, q.p), sx.u) + mulx<13, SOFT>(q.u, sx.p)) +
-               mulx<13, SOFT>(ay, mulx<13, SOFT>(mulx<13, SOFT>(gamma, q.p), sy.v) + mulx<13, SOFT>(q.v, sy.p)));
+  h.r = q.r - ((ax * ((q.u * sx.r) + (q.r * sx.u))) +
+               (ay * ((q.v * sy.r) + (q.r * sy.v))));
+  h.u = q.u - ((ax * ((q.u * sx.u) + fv_div(sx.p, q.r))) + (ay * (q.v * sy.u)));
+  h.v = q.v - ((ax * (q.u * sx.v)) + (ay * ((q.v * sy.v) + fv_div(sy.p, q.r))));
+  h.p = q.p - ((ax * (((gamma * q.p) * sx.u) + (q.u * sx.p))) +
+               (ay * (((gamma * q.p) * sy.v) + (q.v * sy.p))));
+  return h;
+}
+
+template <int SOFT = kSoftMul>
+__device__ __forceinline__ S4<double> hancock(const S4<double> &q, const S4<double> &sx, const S4<double> &sy,
+                                              double ax, double ay, double gamma, const Adder<double> &add) {
+  auto m = [](double a, double b) { return mulx<13, SOFT>(a, b); };
+  S4<double> h;
+  h.r = add.sub(q.r, add(m(ax, add(m(q.u, sx.r), m(q.r, sx.u))), m(ay, add(m(q.v, sy.r), m(q.r, sy.v)))));
+  h.u = add.sub(q.u, add(m(ax, add(m(q.u, sx.u), fv_div(sx.p, q.r))), m(ay, m(q.v, sy.u))));
+  h.v = add.sub(q.v, add(m(ax, m(q.u, sx.v)), m(ay, add(m(q.v, sy.v), fv_div(sy.p, q.r)))));
+  h.p = add.sub(q.p, add(m(ax, add(m(m(gamma, q.p), sx.u), m(q.u, sx.p))),
+                         m(ay, add(m(m(gamma, q.p), sy.v), m(q.v, sy.p)))));
   return h;
 }
 

@@ -50,6 +50,7 @@ struct DevState {
   int error;         // DEVERR_* bit set by a kernel that gave up waiting
   unsigned int ticket;  // CTAs finished in the running launch
   int pad;
+  double one;        // 1.0 (Adder, physics.cuh)
 };
 
 // Constants of the binary32 bound on a cell's inverse dt (physics.cuh).

@@ -141,15 +141,17 @@ struct Smem {
   static constexpr size_t BYTES = sizeof(double) * (TOTAL + 1) + 128;  // + spare slot + alignment slack
 };
 
-// CTAs per SM: 5 of the small tile; 3 of the wide one.  Without viscosity, measured faster with more at the price
-// of register spills (their shared memory still fits): PCM with HLL or HLLC
-// at 5 (40 registers), PCM with FSLP and PLM with HLL or FSLP at 4 (56); PLM
-// and MUSCL-Hancock with HLLC stay at 3.
+// CTAs per SM: 5 of the small tile; 3 of the wide one (72 registers).  Measured
+// faster with more at the price of register spills (their shared memory still
+// fits): PCM with HLLC at 5 (40 registers), with FSLP at 4 (56), PLM with HLL or
+// FSLP at 4 (FSLP RK2 777 x 1501: 0.348 | 0.327 ms a stage at 3 | 4; PCM-HLL
+// 1000 x 600, five steps: 1.39 | 1.43 | 1.48 ms at 3 | 4 | 5; PLM-HLLC KH 2048^2:
+// 1.01 | 1.07 | 1.09 at 3 | 4 | 5).
 template <class T_, int RECON, int RS>
 constexpr int step_ctas_per_sm(bool visc) {
   if (T_::TX < 16) return 5;
   if (visc) return 3;
-  if (RECON == RECON_PCM) return RS == RS_FSLP ? 4 : 5;
+  if (RECON == RECON_PCM) return RS == RS_FSLP ? 4 : RS == RS_HLLC ? 5 : 3;
   if (RECON == RECON_PLM && RS != RS_HLLC) return 4;
   return 3;
 }
@@ -157,9 +159,9 @@ constexpr int step_ctas_per_sm(bool visc) {
 // The products on the integer pipes (physics.cuh): none on small grids, where
 // no pipe is full and a hardware product's latency is a fifth of the
 // integer-pipe one's (Sod 512 x 8: 20.5 -> 18.0 us a step).
-template <class T_>
+template <class T_, int RS>
 __host__ __device__ constexpr int step_soft_mul(bool visc) {
-  return T_::TX < 16 ? 0 : visc ? kSoftMulVisc : kSoftMul;
+  return T_::TX < 16 ? 0 : RS == RS_HLLC ? kSoftMulHllc : visc ? kSoftMulVisc : kSoftMul;
 }
 
 template <class T_, int RECON, int RS, bool VISC>
@@ -168,7 +170,7 @@ __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
                 const StepArgs a) {
   using L = Smem<T_, RECON, VISC>;
   constexpr int TX = T_::TX, TY = T_::TY, SW = T_::SW, SH = T_::SH, NT = T_::NT;
-  constexpr int SOFT = step_soft_mul<T_>(VISC);
+  constexpr int SOFT = step_soft_mul<T_, RS>(VISC);
   // Aligned by offsetting the shared array itself (not through an integer
   // round trip, which would turn every tile access into a generic load).
   extern __shared__ __align__(128) unsigned char fv2d_step_smem[];
@@ -212,7 +214,8 @@ __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
   auto cellQ = [&](int ly, int lx) -> S4<double> {
     return S4<double>{sQ(0, ly, lx), sQ(1, ly, lx), sQ(2, ly, lx), sQ(3, ly, lx)};
   };
-  const Gas<double> gas = make_gas(a.gamma, a.gm1, a.entho, a.fslp_K);
+  const Adder<double> add{*((volatile double *)&st->one)};
+  const Gas<double> gas = make_gas(a.gamma, a.gm1, a.entho, a.fslp_K, add);
 
   // ---- 2. slopes (+ MUSCL-Hancock predictor) and temperatures ------------
   if constexpr (RECON == RECON_PLM) {
@@ -226,12 +229,12 @@ __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
       if (it < NDX) {
         const int k = it / (TY * (TX + 3)), rem = it % (TY * (TX + 3));
         const int ly = rem / (TX + 3) + 2, lx = rem % (TX + 3) + 1;
-        SMI(L::FX + it) = sQ(k, ly, lx) - sQ(k, ly, lx - 1);
+        SMI(L::FX + it) = add.sub(sQ(k, ly, lx), sQ(k, ly, lx - 1));
       } else {
         const int jt = it - NDX;
         const int k = jt / ((TY + 3) * TX), rem = jt % ((TY + 3) * TX);
         const int ly = rem / TX + 1, lx = rem % TX + 2;
-        SMI(L::FX + NDX + jt) = sQ(k, ly, lx) - sQ(k, ly - 1, lx);
+        SMI(L::FX + NDX + jt) = add.sub(sQ(k, ly, lx), sQ(k, ly - 1, lx));
       }
     }
     __syncthreads();
@@ -262,8 +265,8 @@ __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const double c = sQ(k, ly, lx);
-        sR1(L::SX, k, ly, lx) = minmod(c - sQ(k, ly, lx - 1), sQ(k, ly, lx + 1) - c);
-        sR1(L::SY, k, ly, lx) = minmod(c - sQ(k, ly - 1, lx), sQ(k, ly + 1, lx) - c);
+        sR1(L::SX, k, ly, lx) = minmod(add.sub(c, sQ(k, ly, lx - 1)), add.sub(sQ(k, ly, lx + 1), c));
+        sR1(L::SY, k, ly, lx) = minmod(add.sub(c, sQ(k, ly - 1, lx)), add.sub(sQ(k, ly + 1, lx), c));
       }
     }
   }
@@ -286,7 +289,7 @@ __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
       if (ly > ny + 2 || lx > nx + 2) continue;  // past the grid's ghost ring
       S4<double> sx{sR1(L::SX, 0, ly, lx), sR1(L::SX, 1, ly, lx), sR1(L::SX, 2, ly, lx), sR1(L::SX, 3, ly, lx)};
       S4<double> sy{sR1(L::SY, 0, ly, lx), sR1(L::SY, 1, ly, lx), sR1(L::SY, 2, ly, lx), sR1(L::SY, 3, ly, lx)};
-      S4<double> h = hancock<SOFT>(cellQ(ly, lx), sx, sy, ax, ay, a.gamma);
+      S4<double> h = hancock<SOFT>(cellQ(ly, lx), sx, sy, ax, ay, a.gamma, add);
       sR1(L::QH, 0, ly, lx) = h.r;
       sR1(L::QH, 1, ly, lx) = h.u;
       sR1(L::QH, 2, ly, lx) = h.v;
@@ -305,14 +308,14 @@ __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
       const double h0 = sR1(base, 0, ly, lx), h1 = sR1(base, 1, ly, lx), h2 = sR1(base, 2, ly, lx),
                    h3 = sR1(base, 3, ly, lx);
       // q + slope*sign*0.5 (Update.h:25) with the half slope precomputed
-      if (plus) return S4<double>{q.r + h0, q.u + h1, q.v + h2, q.p + h3};
-      return S4<double>{q.r + (-h0), q.u + (-h1), q.v + (-h2), q.p + (-h3)};
+      if (plus) return S4<double>{add(q.r, h0), add(q.u, h1), add(q.v, h2), add(q.p, h3)};
+      return S4<double>{add.sub(q.r, h0), add.sub(q.u, h1), add.sub(q.v, h2), add.sub(q.p, h3)};
     } else {
       const int base = dir ? L::SY : L::SX;
       const double sg = plus ? 1.0 : -1.0;
       S4<double> q{sR1(L::QH, 0, ly, lx), sR1(L::QH, 1, ly, lx), sR1(L::QH, 2, ly, lx), sR1(L::QH, 3, ly, lx)};
-      return S4<double>{q.r + sR1(base, 0, ly, lx) * sg * 0.5, q.u + sR1(base, 1, ly, lx) * sg * 0.5,
-                        q.v + sR1(base, 2, ly, lx) * sg * 0.5, q.p + sR1(base, 3, ly, lx) * sg * 0.5};
+      return S4<double>{add(q.r, sR1(base, 0, ly, lx) * sg * 0.5), add(q.u, sR1(base, 1, ly, lx) * sg * 0.5),
+                        add(q.v, sR1(base, 2, ly, lx) * sg * 0.5), add(q.p, sR1(base, 3, ly, lx) * sg * 0.5)};
     }
   };
 
@@ -375,34 +378,34 @@ __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
         const int ly = r + 2, xs = c + 2, xm = c + 1;
         auto U_ = [&](int dj, int x) { return sQ(1, ly + dj, x); };
         auto V_ = [&](int dj, int x) { return sQ(2, ly + dj, x); };
-        const double qiu = fv_half(U_(0, xs) + U_(0, xm));
-        const double qiv = fv_half(V_(0, xs) + V_(0, xm));
-        const double dudx = mulx<11, SOFT>(odx, U_(0, xs) - U_(0, xm));
-        const double dvdx = mulx<11, SOFT>(odx, V_(0, xs) - V_(0, xm));
-        const double dudy = mulx<11, SOFT>(q_ody, U_(1, xs) - U_(-1, xs) + U_(1, xm) - U_(-1, xm));
-        const double dvdy = mulx<11, SOFT>(q_ody, V_(1, xs) - V_(-1, xs) + V_(1, xm) - V_(-1, xm));
-        const double tau_xx = mulx<11, SOFT>(four_thirds, dudx) - mulx<11, SOFT>(two_thirds, dvdy);
-        const double tau_xy = dvdx + dudy;
+        const double qiu = fv_half(add(U_(0, xs), U_(0, xm)));
+        const double qiv = fv_half(add(V_(0, xs), V_(0, xm)));
+        const double dudx = mulx<11, SOFT>(odx, add.sub(U_(0, xs), U_(0, xm)));
+        const double dvdx = mulx<11, SOFT>(odx, add.sub(V_(0, xs), V_(0, xm)));
+        const double dudy = mulx<11, SOFT>(q_ody, add.sub(add(add.sub(U_(1, xs), U_(-1, xs)), U_(1, xm)), U_(-1, xm)));
+        const double dvdy = mulx<11, SOFT>(q_ody, add.sub(add(add.sub(V_(1, xs), V_(-1, xs)), V_(1, xm)), V_(-1, xm)));
+        const double tau_xx = add.sub(mulx<11, SOFT>(four_thirds, dudx), mulx<11, SOFT>(two_thirds, dvdy));
+        const double tau_xy = add(dvdx, dudy);
         SMI(L::VX + f) = mulx<11, SOFT>(mu, tau_xx);
         SMI(L::VX + f + NVX) = mulx<11, SOFT>(mu, tau_xy);
-        SMI(L::VX + f + 2 * NVX) = mulx<11, SOFT>(mu, mulx<11, SOFT>(tau_xx, qiu) + mulx<11, SOFT>(tau_xy, qiv));
+        SMI(L::VX + f + 2 * NVX) = mulx<11, SOFT>(mu, add(mulx<11, SOFT>(tau_xx, qiu), mulx<11, SOFT>(tau_xy, qiv)));
       } else {  // between rows r+1 (s-1) and r+2 (s) of column c+2
         const int g = f - NVX;
         const int r = g / TX, c = g % TX;
         const int lx = c + 2, ys = r + 2, ym = r + 1;
         auto U_ = [&](int y, int di) { return sQ(1, y, lx + di); };
         auto V_ = [&](int y, int di) { return sQ(2, y, lx + di); };
-        const double qiu = fv_half(U_(ys, 0) + U_(ym, 0));
-        const double qiv = fv_half(V_(ys, 0) + V_(ym, 0));
-        const double dudy = mulx<11, SOFT>(ody, U_(ys, 0) - U_(ym, 0));
-        const double dvdy = mulx<11, SOFT>(ody, V_(ys, 0) - V_(ym, 0));
-        const double dudx = mulx<11, SOFT>(q_odx, U_(ys, 1) - U_(ys, -1) + U_(ym, 1) - U_(ym, -1));
-        const double dvdx = mulx<11, SOFT>(q_odx, V_(ys, 1) - V_(ys, -1) + V_(ym, 1) - V_(ym, -1));
-        const double tau_yy = mulx<11, SOFT>(four_thirds, dvdy) - mulx<11, SOFT>(two_thirds, dudx);
-        const double tau_xy = dvdx + dudy;
+        const double qiu = fv_half(add(U_(ys, 0), U_(ym, 0)));
+        const double qiv = fv_half(add(V_(ys, 0), V_(ym, 0)));
+        const double dudy = mulx<11, SOFT>(ody, add.sub(U_(ys, 0), U_(ym, 0)));
+        const double dvdy = mulx<11, SOFT>(ody, add.sub(V_(ys, 0), V_(ym, 0)));
+        const double dudx = mulx<11, SOFT>(q_odx, add.sub(add(add.sub(U_(ys, 1), U_(ys, -1)), U_(ym, 1)), U_(ym, -1)));
+        const double dvdx = mulx<11, SOFT>(q_odx, add.sub(add(add.sub(V_(ys, 1), V_(ys, -1)), V_(ym, 1)), V_(ym, -1)));
+        const double tau_yy = add.sub(mulx<11, SOFT>(four_thirds, dvdy), mulx<11, SOFT>(two_thirds, dudx));
+        const double tau_xy = add(dvdx, dudy);
         SMI(L::VY + g) = mulx<11, SOFT>(mu, tau_xy);
         SMI(L::VY + g + NVY) = mulx<11, SOFT>(mu, tau_yy);
-        SMI(L::VY + g + 2 * NVY) = mulx<11, SOFT>(mu, mulx<11, SOFT>(tau_xy, qiu) + mulx<11, SOFT>(tau_yy, qiv));
+        SMI(L::VY + g + 2 * NVY) = mulx<11, SOFT>(mu, add(mulx<11, SOFT>(tau_xy, qiu), mulx<11, SOFT>(tau_yy, qiv)));
       }
     }
   }
@@ -419,6 +422,22 @@ __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
   const int P = a.pitch;
   // the dt reduction as other CTAs have left it (any value it has had will do)
   const uint64_t acc = *((volatile unsigned long long *)&st->acc_hyp);
+
+  // x + 0.0; adding dt times (a positive normal number) times +0
+  auto plus_zero = [](double x) { return softfp::bits(x) == softfp::SIGN ? 0.0 : x; };
+  const bool plain = (softfp::bits(dt) >> 52) - 1 < 0x3FF;  // dt positive, normal, below 2
+  // gravity source of one direction (Update.h:165-168).  A zero component (x,
+  // usually) adds zeros, which leave all but a negative zero as it is.
+  auto gravity = [&](double *un, double rho, double F0, double F1, double gv) {
+    auto tame = [](double x) { return softfp::exponent(softfp::bits(x)) < 0x600; };
+    if (softfp::bits(gv) == 0 && plain && softfp::gt0(rho) && tame(rho) && tame(F0) && tame(F1) &&
+        softfp::bits(un[3]) != softfp::SIGN) {
+      un[2] = plus_zero(un[2]);
+    } else {
+      un[2] = add(un[2], dt * rho * gv);
+      un[3] = add(un[3], dt * 0.5 * add(F0, F1) * gv);
+    }
+  };
 
 #pragma unroll 1
   for (int cidx = tid; cidx < TX * TY; cidx += NT) {
@@ -441,15 +460,15 @@ __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
 #pragma unroll
       for (int k = 0; k < 4; k += 2) {
         double d0, d1;
-        mulx2<3, SOFT>(SMI(F + k * S) - SMI(F + k * S + 1), dt, SMI(F + (k + 1) * S) - SMI(F + (k + 1) * S + 1), dt,
+        mulx2<3, SOFT>(add.sub(SMI(F + k * S), SMI(F + k * S + 1)), dt,
+                       add.sub(SMI(F + (k + 1) * S), SMI(F + (k + 1) * S + 1)), dt,
                        d0, d1);
-        un[k] += ddivc(d0, a.dx, a.inv_dx, a.dx_pow2, a.rw_dx);
-        un[k + 1] += ddivc(d1, a.dx, a.inv_dx, a.dx_pow2, a.rw_dx);
+        un[k] = add(un[k], ddivc(d0, a.dx, a.inv_dx, a.dx_pow2, a.rw_dx));
+        un[k + 1] = add(un[k + 1], ddivc(d1, a.dx, a.inv_dx, a.dx_pow2, a.rw_dx));
       }
       if (a.grav_mode) {
         const double gv = (a.grav_mode == 1) ? a.gxf : (double)a.grav_row[j];
-        un[2] += dt * rho * gv;
-        un[3] += dt * 0.5 * (FL0 + FR0) * gv;
+        gravity(un, rho, FL0, FR0, gv);
       }
     }
     // y direction (dir = IY), with the well-balanced boundary override
@@ -477,14 +496,11 @@ __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
 #pragma unroll
       for (int k = 0; k < 4; k += 2) {
         double d0, d1;
-        mulx2<3, SOFT>(FL[k] - FR[k], dt, FL[k + 1] - FR[k + 1], dt, d0, d1);
-        un[k] += ddivc(d0, a.dy, a.inv_dy, a.dy_pow2, a.rw_dy);
-        un[k + 1] += ddivc(d1, a.dy, a.inv_dy, a.dy_pow2, a.rw_dy);
+        mulx2<3, SOFT>(add.sub(FL[k], FR[k]), dt, add.sub(FL[k + 1], FR[k + 1]), dt, d0, d1);
+        un[k] = add(un[k], ddivc(d0, a.dy, a.inv_dy, a.dy_pow2, a.rw_dy));
+        un[k + 1] = add(un[k + 1], ddivc(d1, a.dy, a.inv_dy, a.dy_pow2, a.rw_dy));
       }
-      if (a.grav_mode) {
-        un[2] += dt * rho * gv;
-        un[3] += dt * 0.5 * (FL[0] + FR[0]) * gv;
-      }
+      if (a.grav_mode) gravity(un, rho, FL[0], FR[0], gv);
     }
     // thermal conduction (ThermalConduction.h:46-106)
     if (a.tc) {
@@ -494,8 +510,8 @@ __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
       const double kL = a.kap_row[4 * j + 0], kR = a.kap_row[4 * j + 1];
       const double kU = a.kap_row[4 * j + 2], kD = a.kap_row[4 * j + 3];
       double FLt, FRt, FUt, FDt;
-      mulx2<12, SOFT>(kL, TC - TL, kR, TR - TC, FLt, FRt);
-      mulx2<12, SOFT>(kU, TC - TU, kD, TD - TC, FUt, FDt);
+      mulx2<12, SOFT>(kL, add.sub(TC, TL), kR, add.sub(TR, TC), FLt, FRt);
+      mulx2<12, SOFT>(kU, add.sub(TC, TU), kD, add.sub(TD, TC), FUt, FDt);
       FLt = ddivc(FLt, a.dx, a.inv_dx, a.dx_pow2, a.rw_dx);
       FRt = ddivc(FRt, a.dx, a.inv_dx, a.dx_pow2, a.rw_dx);
       FUt = ddivc(FUt, a.dy, a.inv_dy, a.dy_pow2, a.rw_dy);
@@ -513,8 +529,8 @@ __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
           FRt = kR * a.bctc_ymax_value;
       }
       double dx_part, dy_part;
-      mulx2<12, SOFT>(s_tc[0], FRt - FLt, s_tc[1], FDt - FUt, dx_part, dy_part);
-      un[3] += dx_part + dy_part;
+      mulx2<12, SOFT>(s_tc[0], add.sub(FRt, FLt), s_tc[1], add.sub(FDt, FUt), dx_part, dy_part);
+      un[3] = add(un[3], add(dx_part, dy_part));
     }
     // viscosity (Viscosity.h:63-107): the face terms of the face pass, the
     // -side face negated, accumulated in the reference's order
@@ -522,30 +538,28 @@ __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
       constexpr int NVX = TY * (TX + 1), NVY = (TY + 1) * TX;
       const int Vw = L::VX + ry * (TX + 1) + rx;  // x face at rx (west), rx + 1 (east)
       const int Vn = L::VY + ry * TX + rx;        // y face at ry (north), ry + 1 (south)
-      double fx1 = 0.0, fx2 = 0.0, fx3 = 0.0, fy1 = 0.0, fy2 = 0.0, fy3 = 0.0;
-      fx1 += -SMI(Vw);
-      fx2 += -SMI(Vw + NVX);
-      fx3 += -SMI(Vw + 2 * NVX);
-      fy1 += -SMI(Vn);
-      fy2 += -SMI(Vn + NVY);
-      fy3 += -SMI(Vn + 2 * NVY);
-      fx1 += SMI(Vw + 1);
-      fx2 += SMI(Vw + NVX + 1);
-      fx3 += SMI(Vw + 2 * NVX + 1);
-      fy1 += SMI(Vn + TX);
-      fy2 += SMI(Vn + NVY + TX);
-      fy3 += SMI(Vn + 2 * NVY + TX);
-      un[0] += (0.0 + 0.0) * dt;
+      // 0.0 + (-x) of the reference: -x, and +0 for either zero
+      auto minus = [](double x) {
+        const uint64_t b = softfp::bits(x);
+        return softfp::from_bits((b & softfp::MAG) == 0 ? 0ull : b ^ softfp::SIGN);
+      };
+      const double fx1 = add(minus(SMI(Vw)), SMI(Vw + 1));
+      const double fx2 = add(minus(SMI(Vw + NVX)), SMI(Vw + NVX + 1));
+      const double fx3 = add(minus(SMI(Vw + 2 * NVX)), SMI(Vw + 2 * NVX + 1));
+      const double fy1 = add(minus(SMI(Vn)), SMI(Vn + TX));
+      const double fy2 = add(minus(SMI(Vn + NVY)), SMI(Vn + NVY + TX));
+      const double fy3 = add(minus(SMI(Vn + 2 * NVY)), SMI(Vn + 2 * NVY + TX));
+      un[0] = plain ? plus_zero(un[0]) : un[0] + (0.0 + 0.0) * dt;
       double d1, d2;
-      mulx2<12, SOFT>(fx1 + fy1, dt, fx2 + fy2, dt, d1, d2);
-      un[1] += d1;
-      un[2] += d2;
-      un[3] += mulx<12, SOFT>(fx3 + fy3, dt);
+      mulx2<12, SOFT>(add(fx1, fy1), dt, add(fx2, fy2), dt, d1, d2);
+      un[1] = add(un[1], d1);
+      un[2] = add(un[2], d2);
+      un[3] = add(un[3], mulx<12, SOFT>(add(fx3, fy3), dt));
     }
     // RK2 corrector: 0.5 * (U0 + Unew) (Update.h:214-220)
     if (a.stage == STAGE_RK2_CORRECT) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) un[k] = 0.5 * (a.U[k * PL + g] + un[k]);
+      for (int k = 0; k < 4; ++k) un[k] = fv_half(add(a.U[k * PL + g], un[k]));
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) Udst[k * PL + g] = un[k];
