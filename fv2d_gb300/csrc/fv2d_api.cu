@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(256) prepare_kernel(PrepArgs a) {
   if (threadIdx.x == 0) {
     double m = -1.0;
     for (int w = 0; w < 8; ++w) m = fmax(m, red[w]);
-    if (m >= 0.0) atomicMax(&a.st->acc_hyp, (unsigned long long)__double_as_longlong(m));
+    if (m >= 0.0) atomicMax(&a.st->pending[0].hyp, (unsigned long long)__double_as_longlong(m));
     __threadfence();
     s_last = (atomicAdd(&a.st->ticket, 1u) == (unsigned)a.nblocks - 1u);
   }
@@ -206,17 +206,17 @@ __global__ void __launch_bounds__(256) prepare_kernel(PrepArgs a) {
   if (!s_last || threadIdx.x != 0) return;
   __threadfence();
   volatile DevState *vs = a.st;
-  const double inv_hyp = __longlong_as_double((long long)atomicAdd(&a.st->acc_hyp, 0ull));
+  const double inv_hyp = __longlong_as_double((long long)atomicAdd(&a.st->pending[0].hyp, 0ull));
   double m = inv_hyp;
   if (m < a.inv_tc) m = a.inv_tc;
   if (m < a.inv_visc) m = a.inv_visc;
-  vs->inv_hyp = inv_hyp;
-  vs->dt = a.CFL / m;
+  vs->clock[0].inv_hyp = inv_hyp;
+  vs->clock[0].dt = a.CFL / m;
   for (int k = 0; k < 3; ++k) {
-    vs->counters[k] = 0ull;
-    vs->cnt_acc[k] = 0ull;
+    vs->clock[0].counters[k] = 0ull;
+    vs->pending[0].cnt[k] = 0ull;
   }
-  a.st->acc_hyp = 0ull;
+  a.st->pending[0].hyp = 0ull;
   __threadfence();
   a.st->ticket = 0u;
 }
@@ -243,18 +243,19 @@ __global__ void begin_kernel(DevState *st, double tend, double next_save, double
   st->eps = eps;
   st->check_save = check_save;
   st->max_steps = max_steps;
-  st->steps_in_call = 0;
-  const double t = st->t;
+  Clock &c = st->clock[0];
+  c.steps_in_call = 0;
+  const double t = c.t;
   int s = RUN_RUNNING;
   if (!(t + eps < tend))
     s = RUN_DONE;
   else if (check_save && !skip_first && t + eps > next_save)
     s = RUN_SAVE;
-  else if (!(st->dt > 0.0) || isnan(st->dt) || isinf(st->dt))
+  else if (!(c.dt > 0.0) || isnan(c.dt) || isinf(c.dt))
     s = RUN_NUMERIC;
   else if (max_steps <= 0)
     s = RUN_PAUSED;
-  st->status = s;
+  c.status = s;
 }
 
 int sync_state(fv2d_ctx *ctx) {
@@ -344,12 +345,7 @@ int recon_kind(int r) {
   return RECON_PCM;  // PCM and PCM_WB (Update.h:27-33 falls through to PCM)
 }
 
-int launch_update(fv2d_ctx *ctx, int driven, double dt) {
-  ctx->st_fresh = false;
-  StepArgs a = ctx->args;
-  a.driven = driven;
-  a.dt_arg = dt;
-  a.mirror = driven ? nullptr : ctx->mirror_dev;  // captured device loops never write it
+int launch_stages(fv2d_ctx *ctx, StepArgs &a) {
   const dim3 grid = tile_grid(ctx);
   const int rk = recon_kind(ctx->p.reconstruction);
   if (ctx->p.time_stepping == FV2D_TS_EULER) {
@@ -361,7 +357,42 @@ int launch_update(fv2d_ctx *ctx, int driven, double dt) {
     a.stage = STAGE_RK2_CORRECT;
     CK(launch_step(ctx->tile, ctx->p.riemann_solver, rk, grid, ctx->stream, ctx->tm[0], ctx->tm[1], a));
   }
+  return FV2D_OK;
+}
+
+int launch_update(fv2d_ctx *ctx, double dt) {
+  ctx->st_fresh = false;
+  StepArgs a = ctx->args;
+  a.driven = 0;
+  a.dt_arg = dt;
+  a.mirror = ctx->mirror_dev;
+  if (int rc = launch_stages(ctx, a)) return rc;
   CK(launch_commit(ctx->stream, a));
+  return FV2D_OK;
+}
+
+// n device-driven steps.  Up to kChainedCtas CTAs they are chained: a commit
+// kernel and the gap around it cost ~4 us a step, forming the clock in every
+// CTA's prologue a fraction of one for each wave of CTAs (us a step, commit
+// kernel | chained: KH 64^2 23 | 18, 256^2 37 | 33, 384^2 60 | 58, 640^2 129 | 126,
+// 768^2 as fast, 2048^2 1050 | 1060).  Chained launches also overlap (the next
+// one is dispatched while one runs: 64^2 18 | 17, 352^2 58 | 55), except where
+// their CTAs are one to three to an SM: the early ones crowd on the SMs that have
+// room, and the fullest SM sets the time (256^2, 256 CTAs: 33 | 38).
+constexpr int kChainedCtas = 2048;
+int launch_driven(fv2d_ctx *ctx, int n) {
+  ctx->st_fresh = false;
+  StepArgs a = ctx->args;
+  a.driven = 1;
+  a.mirror = nullptr;  // device loops never write it
+  a.chained = a.nblocks <= kChainedCtas;
+  a.overlapped = a.chained && (ctx->tile == TILE_SMALL ? a.nblocks <= 2 * 152 : a.nblocks > 3 * 152);
+  for (int k = 0; k < n; ++k) {
+    a.step = k;
+    if (int rc = launch_stages(ctx, a)) return rc;
+    a.step = k + 1;
+    if (!a.chained || k + 1 == n) CK(launch_commit(ctx->stream, a));
+  }
   return FV2D_OK;
 }
 
@@ -384,7 +415,7 @@ int run_prepare(fv2d_ctx *ctx, const double *src) {
   PrepArgs pa;
   std::memset(&pa, 0, sizeof(pa));
   pa.q_aos = src;
-  pa.Q = ctx->Q[ctx->st_host->parity];
+  pa.Q = ctx->Q[ctx->st_host->clock[0].parity];
   pa.U = ctx->U;
   pa.st = ctx->st;
   pa.plane = ctx->plane;
@@ -448,8 +479,7 @@ int ensure_graph(fv2d_ctx *ctx) {
   }
   cudaGraph_t g;
   CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-  int rc = FV2D_OK;
-  for (int k = 0; k < G && rc == FV2D_OK; ++k) rc = launch_update(ctx, 1, 0.0);
+  const int rc = launch_driven(ctx, G);
   cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
   if (rc) return rc;
   if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaStreamEndCapture");
@@ -581,7 +611,7 @@ int fv2d_create(const fv2d_params *p, int device, fv2d_ctx **out) {
 
   DevState s0;
   std::memset(&s0, 0, sizeof(s0));
-  s0.status = RUN_PAUSED;
+  s0.clock[0].status = RUN_PAUSED;
   s0.log_cap = ctx->log_cap;
   s0.one = 1.0;
   if ((e = cudaMemcpy(ctx->st, &s0, sizeof(s0), cudaMemcpyHostToDevice)) != cudaSuccess)
@@ -715,14 +745,14 @@ int fv2d_get_prim(fv2d_ctx *ctx, double *q_host) {
   if (!ctx->have_state) return fail(ctx, FV2D_ERR_STATE, "no state: call set_prim or init_problem first");
   if (int rc = sync_state(ctx)) return rc;
   if (ctx->mirror_valid && q_host == ctx->mirror_host) return FV2D_OK;  // the last update wrote it
-  return get_planes(ctx, ctx->Q[ctx->st_host->parity], q_host, cudaMemcpyDeviceToHost);
+  return get_planes(ctx, ctx->Q[ctx->st_host->clock[0].parity], q_host, cudaMemcpyDeviceToHost);
 }
 
 int fv2d_get_prim_device(fv2d_ctx *ctx, double *q_dev) {
   if (!ctx || !q_dev) return FV2D_ERR_INVALID;
   if (!ctx->have_state) return fail(ctx, FV2D_ERR_STATE, "no state: call set_prim or init_problem first");
   if (int rc = sync_state(ctx)) return rc;
-  return get_planes(ctx, ctx->Q[ctx->st_host->parity], q_dev, cudaMemcpyDeviceToDevice);
+  return get_planes(ctx, ctx->Q[ctx->st_host->clock[0].parity], q_dev, cudaMemcpyDeviceToDevice);
 }
 
 int fv2d_get_cons(fv2d_ctx *ctx, double *u_host) {
@@ -736,8 +766,8 @@ int fv2d_compute_dt(fv2d_ctx *ctx, double *dt, double *inv_hyp, double *inv_tc, 
   if (!ctx) return FV2D_ERR_INVALID;
   if (!ctx->have_state) return fail(ctx, FV2D_ERR_STATE, "no state: call set_prim or init_problem first");
   if (int rc = fresh_state(ctx)) return rc;
-  if (dt) *dt = ctx->st_host->dt;
-  if (inv_hyp) *inv_hyp = ctx->st_host->inv_hyp;
+  if (dt) *dt = ctx->st_host->clock[0].dt;
+  if (inv_hyp) *inv_hyp = ctx->st_host->clock[0].inv_hyp;
   if (inv_tc) *inv_tc = ctx->inv_tc;
   if (inv_visc) *inv_visc = ctx->inv_visc;
   return FV2D_OK;
@@ -748,7 +778,7 @@ int fv2d_update(fv2d_ctx *ctx, double dt) {
   if (!ctx) return FV2D_ERR_INVALID;
   if (!ctx->have_state) return fail(ctx, FV2D_ERR_STATE, "no state: call set_prim or init_problem first");
   ctx->mirror_valid = false;
-  if (int rc = launch_update(ctx, 0, dt)) return rc;
+  if (int rc = launch_update(ctx, dt)) return rc;
   ctx->mirror_valid = ctx->mirror_dev != nullptr;
   return FV2D_OK;
 }
@@ -763,23 +793,23 @@ int fv2d_get_device_errors(fv2d_ctx *ctx, int *bits) {
 int fv2d_get_counters(fv2d_ctx *ctx, uint64_t out[3]) {
   if (!ctx || !out) return FV2D_ERR_INVALID;
   if (int rc = sync_state(ctx)) return rc;
-  for (int k = 0; k < 3; ++k) out[k] = ctx->st_host->counters[k];
+  for (int k = 0; k < 3; ++k) out[k] = ctx->st_host->clock[0].counters[k];
   return FV2D_OK;
 }
 
 int fv2d_get_time(fv2d_ctx *ctx, double *t, int *iteration) {
   if (!ctx) return FV2D_ERR_INVALID;
   if (int rc = sync_state(ctx)) return rc;
-  if (t) *t = ctx->st_host->t;
-  if (iteration) *iteration = ctx->st_host->ite;
+  if (t) *t = ctx->st_host->clock[0].t;
+  if (iteration) *iteration = ctx->st_host->clock[0].ite;
   return FV2D_OK;
 }
 
 int fv2d_set_time(fv2d_ctx *ctx, double t, int iteration) {
   if (!ctx) return FV2D_ERR_INVALID;
   if (int rc = sync_state(ctx)) return rc;
-  ctx->st_host->t = t;
-  ctx->st_host->ite = iteration;
+  ctx->st_host->clock[0].t = t;
+  ctx->st_host->clock[0].ite = iteration;
   CK(cudaMemcpyAsync(ctx->st, ctx->st_host, sizeof(DevState), cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   return FV2D_OK;
@@ -808,9 +838,9 @@ int fv2d_advance(fv2d_ctx *ctx, int max_steps, double tend, double next_save, in
       launched += G;
     }
     if (int rc = sync_state(ctx)) return rc;
-    if (ctx->st_host->status != RUN_RUNNING || launched >= max_steps) break;
+    if (ctx->st_host->clock[0].status != RUN_RUNNING || launched >= max_steps) break;
   }
-  const DevState &s = *ctx->st_host;
+  const Clock &s = ctx->st_host->clock[0];
   if (t) *t = s.t;
   if (steps_done) *steps_done = s.steps_in_call;
   int out = FV2D_RUN_STEPS;
@@ -818,7 +848,7 @@ int fv2d_advance(fv2d_ctx *ctx, int max_steps, double tend, double next_save, in
   else if (s.status == RUN_SAVE) out = FV2D_RUN_SAVE;
   else if (s.status == RUN_NUMERIC) out = FV2D_RUN_NUMERIC;
   if (status) *status = out;
-  if (s.error) return fail(ctx, FV2D_ERR_CUDA, "a step kernel timed out waiting for its tile load");
+  if (ctx->st_host->error) return fail(ctx, FV2D_ERR_CUDA, "a step kernel timed out waiting for its tile load");
   return out == FV2D_RUN_NUMERIC ? fail(ctx, FV2D_ERR_NUMERIC, "non-finite or non-positive dt") : FV2D_OK;
 }
 
@@ -833,15 +863,13 @@ int fv2d_run_async(fv2d_ctx *ctx, int n) {
   if (int rc = ensure_graph(ctx)) return rc;
   long long k = 0;
   for (; k + ctx->graph_steps <= n; k += ctx->graph_steps) CK(cudaGraphLaunch(ctx->graph, ctx->stream));
-  for (; k < n; ++k)
-    if (int rc = launch_update(ctx, 1, 0.0)) return rc;
-  return FV2D_OK;
+  return launch_driven(ctx, (int)(n - k));
 }
 
 int fv2d_get_step_log(fv2d_ctx *ctx, double *records, int max_records, int *count) {
   if (!ctx || !records || max_records < 0) return FV2D_ERR_INVALID;
   if (int rc = sync_state(ctx)) return rc;
-  int n = std::min(std::min(ctx->st_host->steps_in_call, ctx->log_cap), max_records);
+  int n = std::min(std::min(ctx->st_host->clock[0].steps_in_call, ctx->log_cap), max_records);
   if (n > 0) {
     CK(cudaMemcpyAsync(records, ctx->log, sizeof(double) * 6 * n, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));

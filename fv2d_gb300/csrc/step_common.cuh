@@ -28,29 +28,44 @@ enum { STAGE_EULER = 0, STAGE_RK2_PREDICT = 1, STAGE_RK2_CORRECT = 2 };
 enum { RUN_RUNNING = 0, RUN_DONE = 1, RUN_SAVE = 2, RUN_NUMERIC = 3, RUN_PAUSED = 4 };
 enum { DEVERR_TMA_TIMEOUT = 1, DEVERR_BOUNDS = 2 };
 
-// Simulation clock, dt and reduction accumulators, resident in device memory.
-// Written by the last CTA of each step (or by the set-up pass), read by the
-// next launch: kernels never exchange these within a launch.
-struct DevState {
+// The simulation clock: what a committed step leaves behind.
+struct Clock {
   double t;          // time after the last committed update (main.cpp:83)
   double dt;         // CFL dt of the current primitive state (ComputeDt.h:64)
   double inv_hyp;    // max inverse hyperbolic dt of the current state
   double last_dt;    // dt used by the last update
-  double tend, next_save, eps;  // device-driven loop control
-  unsigned long long acc_hyp;   // running max (bits of a non-negative double)
-  unsigned long long cnt_acc[3];
   unsigned long long counters[3];  // checkNegatives counts of the last update
   int parity;        // which primitive buffer holds the current state
   int ite;           // committed updates
   int status;        // RUN_*
-  int check_save;    // stop before an iteration that must write a snapshot
   int steps_in_call; // iterations done by the current fv2d_advance
+};
+
+// Reductions of a step that is not committed yet.
+struct StepSums {
+  unsigned long long hyp;  // running max of the inverse hyperbolic dt (bits of a non-negative double)
+  unsigned long long cnt[3];
+};
+
+// Clock, reductions and loop control, resident in device memory.  Between
+// calls clock[0] is the state and every StepSums is zero.  A step followed by
+// commit_kernel reduces into pending[0], which that kernel commits to clock[0].
+// In a chained sequence (StepArgs::chained) step k commits step k - 1 itself: its
+// CTAs all form the new clock from clock[k & 1] and pending[(k - 1) & 3], one
+// of them stores it in clock[(k + 1) & 1] and clears pending[(k + 1) & 3] (last
+// read two launches ago), and they reduce into pending[k & 3]; commit_kernel
+// ends the sequence.  No launch writes what another CTA of it reads.
+struct DevState {
+  Clock clock[2];
+  StepSums pending[4];
+  double tend, next_save, eps;  // device-driven loop control
+  double one;        // 1.0 (Adder, physics.cuh)
+  int check_save;    // stop before an iteration that must write a snapshot
   int max_steps;     // iteration cap of the current fv2d_advance
   int log_cap;       // capacity of the per-iteration log (records)
   int error;         // DEVERR_* bit set by a kernel that gave up waiting
-  unsigned int ticket;  // CTAs finished in the running launch
+  unsigned int ticket;  // CTAs of the set-up pass that finished
   int pad;
-  double one;        // 1.0 (Adder, physics.cuh)
 };
 
 // Constants of the binary32 bound on a cell's inverse dt (physics.cuh).
@@ -73,6 +88,9 @@ struct StepArgs {
   int nblocks;
   int stage;          // STAGE_*
   int driven;         // 1: dt and loop control from DevState
+  int chained;        // 1: step `step` of a sequence that commits its own steps
+  int step;
+  int overlapped;     // 1: dispatched while the previous launch runs
   double dt_arg;      // dt when driven == 0
   // gas and mesh constants
   double gamma, gm1, entho, fslp_K;

@@ -164,6 +164,60 @@ __host__ __device__ constexpr int step_soft_mul(bool visc) {
   return T_::TX < 16 ? 0 : RS == RS_HLLC ? kSoftMulHllc : visc ? kSoftMulVisc : kSoftMul;
 }
 
+// The clock after a step: t += dt, the counters, the next dt, and the
+// device-driven loop condition (main.cpp:62-64, 83; ComputeDt.h:64).
+__device__ __forceinline__ Clock committed(const StepArgs &a, const Clock &c, const StepSums &p) {
+  const volatile DevState *st = a.st;
+  const double dt = a.driven ? c.dt : a.dt_arg;
+  const double inv_hyp = __longlong_as_double((long long)p.hyp);
+  double m = inv_hyp;  // std::max({hyp, tc, visc}) (ComputeDt.h:64)
+  if (m < a.inv_tc) m = a.inv_tc;
+  if (m < a.inv_visc) m = a.inv_visc;
+  Clock n = c;
+  n.t = c.t + dt;
+  n.last_dt = dt;
+  n.inv_hyp = inv_hyp;
+  n.dt = fv_div(a.CFL, m);
+  n.ite = c.ite + 1;
+  if (a.stage == STAGE_EULER) n.parity = 1 - c.parity;
+  for (int k = 0; k < 3; ++k) n.counters[k] = p.cnt[k];
+  n.steps_in_call = c.steps_in_call + 1;
+  if (a.driven) {
+    int s = RUN_RUNNING;
+    if (!(n.t + st->eps < st->tend))
+      s = RUN_DONE;  // main.cpp:62
+    else if (st->check_save && n.t + st->eps > st->next_save)
+      s = RUN_SAVE;  // main.cpp:64
+    else if (!(n.dt > 0.0) || isnan(n.dt) || isinf(n.dt))
+      s = RUN_NUMERIC;
+    else if (n.steps_in_call >= st->max_steps)
+      s = RUN_PAUSED;
+    n.status = s;
+  }
+  return n;
+}
+// The log record of the step that took clock c to n.
+__device__ __forceinline__ void log_step(const StepArgs &a, const Clock &c, const Clock &n) {
+  if (!a.log || c.steps_in_call >= a.st->log_cap) return;
+  double *rec = a.log + 6 * c.steps_in_call;
+  rec[0] = c.t;
+  rec[1] = n.last_dt;
+  rec[2] = c.inv_hyp;
+  rec[3] = (double)n.counters[0];
+  rec[4] = (double)n.counters[1];
+  rec[5] = (double)n.counters[2];
+}
+// A copy through L2 of a structure of 8-byte words that this launch does not write.
+template <class T>
+__device__ __forceinline__ T load_words(const T *p) {
+  T v;
+  const unsigned long long *w = reinterpret_cast<const unsigned long long *>(p);
+  unsigned long long *o = reinterpret_cast<unsigned long long *>(&v);
+#pragma unroll
+  for (int k = 0; k < (int)(sizeof(T) / 8); ++k) o[k] = __ldcg(w + k);
+  return v;
+}
+
 template <class T_, int RECON, int RS, bool VISC>
 __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
     step_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant__ CUtensorMap tmQ1,
@@ -180,29 +234,57 @@ __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
   __shared__ double s_tc[2];  // dt/dx, dt/dy of the conduction update (ThermalConduction.h:106), once per CTA
   __shared__ unsigned red_cnt[3][NT / 32];
 
+  __shared__ struct {
+    double dt;
+    int parity, run;
+  } now;
+
   DevState *st = a.st;
   const int tid = threadIdx.x;
-  if (a.driven && *((volatile int *)&st->status) != RUN_RUNNING) return;
-  const int par = *((volatile int *)&st->parity);
-  const double dt = a.driven ? *((volatile double *)&st->dt) : a.dt_arg;
-  const int src = (a.stage == STAGE_RK2_CORRECT) ? 1 - par : par;
-  const int dst = 1 - src;
-  const CUtensorMap *tm = src ? &tmQ1 : &tmQ0;
-
   const int bx = blockIdx.x, by = blockIdx.y;
   const int i0 = bx * TX, j0 = by * TY;  // first interior cell of the tile
   const int nx = min(TX, a.Nx - i0), ny = min(TY, a.Ny - j0);  // its cells inside the grid
 
-  // ---- 1. stage tile + halo (padded coordinates start at the halo) -------
+  // ---- 1. the clock; stage tile + halo (padded coordinates start at the halo)
+  // A chained launch is dispatched while the previous one runs: everything it
+  // reads or writes comes after this wait for that launch's end (which
+  // returns at once in a launch dispatched in plain stream order).
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (tid == 0) {
     mbar_init(&mbar, 1);
     fence_mbar_init();
+    const bool corrects = a.stage == STAGE_RK2_CORRECT;
+    // of a chained sequence, the corrector's clock is the one its predictor stored
+    const int from = !a.chained ? 0 : (a.step + corrects) & 1;
+    Clock c = load_words(&st->clock[from]);
+    const bool commits = a.chained && a.step > 0 && !corrects && c.status == RUN_RUNNING;
+    const int par = commits && a.stage == STAGE_EULER ? 1 - c.parity : c.parity;
+    const int src = corrects ? 1 - par : par;
+    // the load needs the parity alone: the rest of the clock is formed behind it
+    mbar_expect_tx(&mbar, 4u * SH * SW * sizeof(double));
+    tma_load_3d(sm + L::Q, src ? &tmQ1 : &tmQ0, i0, j0, 0, &mbar);
+    if (a.chained && !corrects) {
+      const Clock before = c;
+      if (commits) c = committed(a, c, load_words(&st->pending[(a.step + 3) & 3]));
+      if (bx == 0 && by == 0) {
+        if (commits) log_step(a, before, c);
+        st->clock[(a.step + 1) & 1] = c;
+        st->pending[(a.step + 1) & 3] = StepSums{0ull, {0ull, 0ull, 0ull}};
+      }
+    }
+    now.dt = a.driven ? c.dt : a.dt_arg;
+    now.parity = par;
+    now.run = !a.driven || c.status == RUN_RUNNING;
   }
   __syncthreads();
-  if (tid == 0) {
-    mbar_expect_tx(&mbar, 4u * SH * SW * sizeof(double));
-    tma_load_3d(sm + L::Q, tm, i0, j0, 0, &mbar);
+  if (!now.run) {
+    if (tid == 0) mbar_wait_bounded(&mbar, &st->error);
+    return;
   }
+  const double dt = now.dt;
+  const int dst = (a.stage == STAGE_RK2_CORRECT) ? now.parity : 1 - now.parity;
+  StepSums *pending = &st->pending[a.chained ? a.step & 3 : 0];
   mbar_wait_bounded(&mbar, &st->error);
 
   auto SMI = [&](int i) -> double & { return sm[smem_index(i, L::TOTAL, &st->error)]; };
@@ -421,7 +503,7 @@ __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
   const long long PL = a.plane;
   const int P = a.pitch;
   // the dt reduction as other CTAs have left it (any value it has had will do)
-  const uint64_t acc = *((volatile unsigned long long *)&st->acc_hyp);
+  const uint64_t acc = *((volatile unsigned long long *)&pending->hyp);
 
   // x + 0.0; adding dt times (a positive normal number) times +0
   auto plus_zero = [](double x) { return softfp::bits(x) == softfp::SIGN ? 0.0 : x; };
@@ -635,68 +717,25 @@ __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
     }
     // reductions only (no value returned, no fence): the commit kernel that
     // follows in stream order reads the totals
-    if (m >= 0.0) atomicMax(&st->acc_hyp, (unsigned long long)__double_as_longlong(m));
-    if (c0) atomicAdd(&st->cnt_acc[0], (unsigned long long)c0);
-    if (c1) atomicAdd(&st->cnt_acc[1], (unsigned long long)c1);
-    if (c2) atomicAdd(&st->cnt_acc[2], (unsigned long long)c2);
+    if (m >= 0.0) atomicMax(&pending->hyp, (unsigned long long)__double_as_longlong(m));
+    if (c0) atomicAdd(&pending->cnt[0], (unsigned long long)c0);
+    if (c1) atomicAdd(&pending->cnt[1], (unsigned long long)c1);
+    if (c2) atomicAdd(&pending->cnt[2], (unsigned long long)c2);
   }
 }
 
-// ---- 6. commit the step (one thread, after the step kernel in stream order):
-// t += dt, the counters, the next dt, the per-iteration log and the
-// device-driven loop condition (main.cpp:62-64, 83; ComputeDt.h:64).
+// ---- 6. commit the step (one thread, after the step kernel in stream order),
+// or the last step of a chained sequence of a.step steps.
 static __global__ void commit_kernel(const StepArgs a) {
   DevState *st = a.st;
-  volatile DevState *vs = st;
-  if (a.driven && vs->status != RUN_RUNNING) return;
-  const int par = vs->parity;
-  const double dt = a.driven ? vs->dt : a.dt_arg;
-  const double inv_prev = vs->inv_hyp;
-  const double t_before = vs->t;
-  const double inv_hyp = __longlong_as_double((long long)vs->acc_hyp);
-  double m = inv_hyp;  // std::max({hyp, tc, visc}) (ComputeDt.h:64)
-  if (m < a.inv_tc) m = a.inv_tc;
-  if (m < a.inv_visc) m = a.inv_visc;
-  const double dt_next = a.CFL / m;
-  const double t_after = t_before + dt;
-  vs->t = t_after;
-  vs->last_dt = dt;
-  vs->inv_hyp = inv_hyp;
-  vs->dt = dt_next;
-  const int ite = vs->ite;
-  vs->ite = ite + 1;
-  if (a.stage == STAGE_EULER) vs->parity = 1 - par;
-  unsigned long long cnt[3];
-  for (int k = 0; k < 3; ++k) {
-    cnt[k] = vs->cnt_acc[k];
-    vs->counters[k] = cnt[k];
-    st->cnt_acc[k] = 0ull;
+  const Clock c = load_words(&st->clock[a.chained ? a.step & 1 : 0]);
+  Clock n = c;
+  if (!a.driven || c.status == RUN_RUNNING) {
+    n = committed(a, c, load_words(&st->pending[a.chained ? (a.step + 3) & 3 : 0]));
+    log_step(a, c, n);
   }
-  st->acc_hyp = 0ull;
-  const int n = vs->steps_in_call;
-  if (a.log && n < vs->log_cap) {
-    double *rec = a.log + 6 * n;
-    rec[0] = t_before;
-    rec[1] = dt;
-    rec[2] = inv_prev;
-    rec[3] = (double)cnt[0];
-    rec[4] = (double)cnt[1];
-    rec[5] = (double)cnt[2];
-  }
-  vs->steps_in_call = n + 1;
-  if (a.driven) {
-    int s = RUN_RUNNING;
-    if (!(t_after + vs->eps < vs->tend))
-      s = RUN_DONE;  // main.cpp:62
-    else if (vs->check_save && t_after + vs->eps > vs->next_save)
-      s = RUN_SAVE;  // main.cpp:64
-    else if (!(dt_next > 0.0) || isnan(dt_next) || isinf(dt_next))
-      s = RUN_NUMERIC;
-    else if (n + 1 >= vs->max_steps)
-      s = RUN_PAUSED;
-    vs->status = s;
-  }
+  st->clock[0] = n;
+  for (int k = 0; k < (a.chained ? 4 : 1); ++k) st->pending[k] = StepSums{0ull, {0ull, 0ull, 0ull}};
 }
-
 
 }  // namespace fv2d

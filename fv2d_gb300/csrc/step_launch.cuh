@@ -28,33 +28,40 @@ cudaError_t set_step_attrs() {
   return e;
 }
 
+template <class T, int RECON, int RS, bool VISC>
+cudaError_t launch_step_one(dim3 grid, cudaStream_t s, const CUtensorMap &t0, const CUtensorMap &t1,
+                            const StepArgs &a) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(T::NT);
+  cfg.dynamicSmemBytes = Smem<T, RECON, VISC>::BYTES;
+  cfg.stream = s;
+  cudaLaunchAttribute overlap = {};
+  overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  overlap.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &overlap;
+  cfg.numAttrs = a.overlapped ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, step_kernel<T, RECON, RS, VISC>, t0, t1, a);
+}
+
 template <class T, int RS, bool VISC>
-void launch_step_recon(int recon, dim3 grid, cudaStream_t s, const CUtensorMap &t0, const CUtensorMap &t1,
-                       const StepArgs &a) {
+cudaError_t launch_step_recon(int recon, dim3 grid, cudaStream_t s, const CUtensorMap &t0, const CUtensorMap &t1,
+                              const StepArgs &a) {
   switch (recon) {
-    case RECON_PLM:
-      step_kernel<T, RECON_PLM, RS, VISC><<<grid, T::NT, Smem<T, RECON_PLM, VISC>::BYTES, s>>>(t0, t1, a);
-      break;
-    case RECON_MH:
-      step_kernel<T, RECON_MH, RS, VISC><<<grid, T::NT, Smem<T, RECON_MH, VISC>::BYTES, s>>>(t0, t1, a);
-      break;
-    default:
-      step_kernel<T, RECON_PCM, RS, VISC><<<grid, T::NT, Smem<T, RECON_PCM, VISC>::BYTES, s>>>(t0, t1, a);
-      break;
+    case RECON_PLM: return launch_step_one<T, RECON_PLM, RS, VISC>(grid, s, t0, t1, a);
+    case RECON_MH: return launch_step_one<T, RECON_MH, RS, VISC>(grid, s, t0, t1, a);
+    default: return launch_step_one<T, RECON_PCM, RS, VISC>(grid, s, t0, t1, a);
   }
 }
 
 template <int RS>
 cudaError_t launch_step_rs(int tile, int recon, dim3 grid, cudaStream_t s, const CUtensorMap &t0,
                            const CUtensorMap &t1, const StepArgs &a) {
-  if (tile == TILE_SMALL) {
-    if (a.visc) launch_step_recon<SmallTile, RS, true>(recon, grid, s, t0, t1, a);
-    else launch_step_recon<SmallTile, RS, false>(recon, grid, s, t0, t1, a);
-  } else {
-    if (a.visc) launch_step_recon<WideTile, RS, true>(recon, grid, s, t0, t1, a);
-    else launch_step_recon<WideTile, RS, false>(recon, grid, s, t0, t1, a);
-  }
-  return cudaGetLastError();
+  if (tile == TILE_SMALL)
+    return a.visc ? launch_step_recon<SmallTile, RS, true>(recon, grid, s, t0, t1, a)
+                  : launch_step_recon<SmallTile, RS, false>(recon, grid, s, t0, t1, a);
+  return a.visc ? launch_step_recon<WideTile, RS, true>(recon, grid, s, t0, t1, a)
+                : launch_step_recon<WideTile, RS, false>(recon, grid, s, t0, t1, a);
 }
 
 }  // namespace fv2d
