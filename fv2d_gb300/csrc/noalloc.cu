@@ -74,7 +74,7 @@ __device__ __forceinline__ double div_spacing(double x, double d, double inv_d, 
 // cell): each thread takes the binary32 upper bound (physics.cuh) of its 16
 // cells from one pass over them, and only the cells whose bound is within the
 // bounds' slack of the CTA's largest are evaluated exactly (a second read,
-// from L2).  Evaluating every cell exactly took 109 us on 3000 x 2000 cells,
+// from L2).  Evaluating every cell exactly took 109 us,
 // against 28 us of HBM time.
 __global__ void __launch_bounds__(kThreads) dt_noalloc_kernel(DtArgs a) {
   __shared__ double red[kThreads / 32];
@@ -107,17 +107,16 @@ __global__ void __launch_bounds__(kThreads) dt_noalloc_kernel(DtArgs a) {
   for (int w = 0; w < kThreads / 32; ++w) top = fmaxf(top, redf[w]);
   // a bound is less than 1 + 2^-17 times its value: a cell below this
   // threshold is below the value of the cell with the largest bound
-  const float least = top * (1.0f - 0x1p-16f);
-  double m = -1.0;
-#pragma unroll 1
-  for (int k = 0; k < kCellsPerThread; ++k) {
-    const long long c = base + (long long)k * kThreads + threadIdx.x;
-    float b = bound[0];
+  const float least = fmaxf(top * (1.0f - 0x1p-16f), 0.f);
+  unsigned todo = 0;
 #pragma unroll
-    for (int j = 1; j < kCellsPerThread; ++j) b = j == k ? bound[j] : b;
-    if (c < a.ncells && !(b < least)) {
-      const fv2d::Gas<double> gas = fv2d::make_gas(a.gamma, a.gm1, 1.0 / a.gm1, 0.0);
-      const fv2d::S4<double> q = cell(c);
+  for (int k = 0; k < kCellsPerThread; ++k)
+    todo |= bound[k] < least ? 0u : 1u << k;  // a cell past the end has bound -1
+  double m = -1.0;
+  if (todo) {
+    const fv2d::Gas<double> gas = fv2d::make_gas(a.gamma, a.gm1, 1.0 / a.gm1, 0.0);
+    for (; todo; todo &= todo - 1) {
+      const fv2d::S4<double> q = cell(base + (long long)(__ffs(todo) - 1) * kThreads + threadIdx.x);
       const double cs = fv2d::sound_speed(q, gas);
       const double ih = div_spacing(cs + fabs(q.u), a.dx, a.inv_dx, a.dx_pow2, a.rw_dx) +
                         div_spacing(cs + fabs(q.v), a.dy, a.inv_dy, a.dy_pow2, a.rw_dy);
