@@ -70,25 +70,32 @@ inline int choose_band(const std::vector<BandGrid> &grids, double resident_warps
   return kMinBand;
 }
 
-// Band height of a march lane that can run in one wave: the shortest that gives
-// it no more items than the resident warps, or 0 when that takes bands taller
-// than kMaxWaveBand (choose_band then picks).  A lane with fewer items than warps
-// is bound by the chain of a work item's rows (1.4 us a row, 4 rows of window
-// fill beside the band's), not by throughput, so shorter bands shorten the step
-// until the warps are used up; and at 8 to 12 rows one full wave beats the next
-// shorter band's wave and a bit.  Measured, ms per 100 steps, choose_band | this:
-// KH 128^2 2.03 | 1.11, 256^2 2.07 | 1.06, 512^2 2.20 | 1.52; RT 128 x 384
-// 1.77 | 1.23, 512 x 1536 3.46 | 3.09 (10 rows).  Several such lanes side by side
-// do best with every lane sized as if alone (16 mixed grids: 5.63 against 6.08
-// with the warps shared out).  Where a full wave needs taller bands the plentiful
-// items of choose_band are as good (KH 2048^2: 30 rows 17.4, 12 rows 18.0).
-constexpr int kMaxWaveBand = 12;
+// Band height of a march lane that can run in one or two full waves: the
+// shortest that gives it no more items than the resident warps, up to
+// kOneWaveBand rows, else than twice as many, up to kTwoWaveBand rows, else 0
+// (choose_band then picks).  A lane with fewer items than warps is bound by the
+// chain of a work item's rows (1.4 us a row, 4 rows of window fill beside the
+// band's), not by throughput, so shorter bands shorten the step until the warps
+// are used up; and a full wave or two beat the next shorter band's wave and a
+// bit.  Measured, ms per 100 steps, choose_band | this: KH 128^2 2.03 | 1.11,
+// 256^2 2.07 | 1.06, 512^2 2.20 | 1.52, 1000 x 2000 5.50 | 5.10 (14 rows),
+// 2048^2 10.4 | 9.6 (two waves of 15 rows); RT 128 x 384 1.77 | 1.23,
+// 512 x 1536 3.46 | 3.09 (10 rows), 1400^2 6.67 | 6.42 (two waves of 12).
+// Taller full waves than these are no better than choose_band's plentiful items
+// (KH 2048^2: one wave of 30 rows 10.0).  Several such lanes side by side do
+// best with every lane sized as if alone (16 mixed grids: 5.63 against 6.08 with
+// the warps shared out).
+constexpr int kOneWaveBand = 18, kTwoWaveBand = 16;
 inline int choose_wave_band(const std::vector<BandGrid> &grids, double warps) {
-  for (int H = 1; H <= kMaxWaveBand; ++H) {
-    double items = 0;
-    for (const BandGrid &g : grids) items += (double)g.strips * ((g.Ny + H - 1) / H);
-    if (items <= warps) return H;
-  }
+  auto items = [&](int H) {
+    double n = 0;
+    for (const BandGrid &g : grids) n += (double)g.strips * ((g.Ny + H - 1) / H);
+    return n;
+  };
+  for (int H = 1; H <= kOneWaveBand; ++H)
+    if (items(H) <= warps) return H;
+  for (int H = kMinBand; H <= kTwoWaveBand; ++H)
+    if (items(H) <= 2 * warps) return H;
   return 0;
 }
 

@@ -1,6 +1,6 @@
-"""The one-wave band height of the service's march lanes, on the host against a
-restatement: the shortest of 1..12 rows whose work items fit the resident
-warps, 0 when none does."""
+"""The full-wave band height of the service's march lanes, on the host against a
+restatement: the shortest of 1..18 rows whose work items fit the resident
+warps, else of 8..16 rows whose items fit them twice over, else 0."""
 import os
 import shutil
 import subprocess
@@ -12,9 +12,10 @@ from fv2d_testlib import REPO
 
 
 def rule(grids, warps):
-    for H in range(1, 13):
-        if sum(s * -(-ny // H) for s, ny in grids) <= warps:
-            return H
+    for waves, heights in ((1, range(1, 19)), (2, range(8, 17))):
+        for H in heights:
+            if sum(s * -(-ny // H) for s, ny in grids) <= waves * warps:
+                return H
     return 0
 
 
@@ -26,10 +27,10 @@ def test_wave_band_matches_the_rule(tmp_path):
     subprocess.run([cxx, "-std=c++17", "-O2", "-Wall", "-Werror", "-o", exe,
                     os.path.join(REPO, "tests", "schedule_wave_harness.cpp")], check=True)
     rng = np.random.default_rng(3)
-    # lone grids: 128^2 a row an item, 512^2 two, RT 512 x 1536 ten, 2048^2 none
+    # lone grids: 128^2 a row an item, 512^2 two, RT 512 x 1536 ten, 2048^2 two waves of 15, 4096^2 none
     cases = [([(3, 128)], 2432.0), ([(9, 512)], 2432.0), ([(19, 1536)], 3040.0), ([(35, 2048)], 2432.0),
-             ([(1, 12)], 1.0), ([(1, 13)], 1.0)]
-    expect = [1, 2, 10, 0, 12, 0]
+             ([(69, 4096)], 2432.0), ([(1, 18)], 1.0), ([(1, 19)], 1.0), ([(1, 33)], 1.0)]
+    expect = [1, 2, 10, 15, 0, 18, 10, 0]
     for _ in range(300):
         n = int(rng.integers(1, 30))
         cases.append(([(int(rng.integers(1, 40)), int(rng.integers(16, 1500))) for _ in range(n)],
