@@ -98,6 +98,12 @@ __device__ __forceinline__ float pressure_of(float dE, float bg_e, float r, floa
   return __fmul_rn(__fadd_rn(__fsub_rn(dE, ek), bg_e), gm1);
 }
 
+// the smaller of the two, NaN when either is
+__device__ __forceinline__ float min_nan(float a, float b) {
+  float m;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
+  return m;
+}
 __device__ __forceinline__ bool is_nan_f(float x) { return (__float_as_uint(x) & 0x7FFFFFFFu) > 0x7F800000u; }
 
 // A work item of one simulation: sim index in the table, item coordinates.

@@ -18,9 +18,10 @@ static const BatchCfg kMarch2[] = {
     // named <strip columns>/<threads per CTA>x<CTAs per SM>/march2[-diff]
     FV2D_MARCH2(32, 32, 16, "60/32x16/march2"),
     FV2D_MARCH2(32, 32, 12, "60/32x12/march2"),
-    // the diffusive body measured slower than the one-column march on the
-    // Rayleigh-Taylor set-up (31.8 against 37.2 G cell-updates/s at
-    // 1024 x 3072); kept as a candidate for other devices and mixes
+    // the diffusive body: 16 CTAs per SM where the lane then runs in fewer
+    // waves (RT 1400^2, ms per 100 steps: 5.54 | 6.25 at 10), 10 elsewhere
+    // (RT 1024 x 3072 8.75 | 8.59, 128 x 384 1.22 | 1.19)
+    FV2D_MARCH2_DIFF(32, 32, 16, "60/32x16/march2-diff"),
     FV2D_MARCH2_DIFF(32, 32, 10, "60/32x10/march2-diff"),
 };
 

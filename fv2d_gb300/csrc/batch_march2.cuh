@@ -66,12 +66,12 @@ __device__ __forceinline__ f2 right(f2 a) { return make_float2(a.y, __shfl_down_
 __device__ __forceinline__ Q2 left(const Q2 &q) { return Q2{left(q.r), left(q.u), left(q.v), left(q.p)}; }
 __device__ __forceinline__ Q2 right(const Q2 &q) { return Q2{right(q.r), right(q.u), right(q.v), right(q.p)}; }
 
-// minmod (Update.h:77-85) of each column's left and right differences
+// minmod (Update.h:77-85) of each column's left and right differences as the
+// median of the two and zero: four minima and maxima a column, where the
+// product's sign took two comparisons, two selects and the product (and missed
+// opposite signs whose product underflows)
 __device__ __forceinline__ f2 minmod2(f2 dl, f2 dr) {
-  const f2 prod = dl * dr;
-  const float mx = fabsf(dl.x) < fabsf(dr.x) ? dl.x : dr.x;
-  const float my = fabsf(dl.y) < fabsf(dr.y) ? dl.y : dr.y;
-  return make_float2(prod.x < 0.f ? 0.f : mx, prod.y < 0.f ? 0.f : my);
+  return max2(min2(dl, dr), min2(max2(dl, dr), F2(0.f)));
 }
 __device__ __forceinline__ Q2 slope(const Q2 &dl, const Q2 &dr) {
   return Q2{minmod2(dl.r, dr.r), minmod2(dl.u, dr.u), minmod2(dl.v, dr.v), minmod2(dl.p, dr.p)};
@@ -120,15 +120,15 @@ __device__ __forceinline__ void hll(const Q2 &qL, const Q2 &qR, Q2 &f, f2 &pout,
 }
 
 // RiemannSolvers.h:53-128: the star state of the side the reference would
-// reach (u* > 0 -> left), then the final state in its branch order.
+// reach (u* > 0 -> left), then the final state in its branch order.  The side
+// K is picked once (SL > 0 takes the left state whatever u* is), so every
+// select below serves the star state and the flux (18 of them instead of 32),
+// the total energy is formed for that side only, and the larger sound speed is
+// the root of the larger square.
 __device__ __forceinline__ void hllc(const Q2 &qL, const Q2 &qR, Q2 &f, f2 &pout, const Gas2 &g) {
   const f2 rL = qL.r, uL = qL.u, vL = qL.v, pL = qL.p;
   const f2 rR = qR.r, uR = qR.u, vR = qR.v, pR = qR.p;
-  const f2 EL = fma2(g.half * rL, fma2(uL, uL, vL * vL), pL * g.entho);
-  const f2 ER = fma2(g.half * rR, fma2(uR, uR, vR * vR), pR * g.entho);
-  const f2 cL = sqrt2(pL * g.gamma * rcp2(rL));
-  const f2 cR = sqrt2(pR * g.gamma * rcp2(rR));
-  const f2 cmax = max2(cL, cR);
+  const f2 cmax = sqrt2(max2(pL * g.gamma * rcp2(rL), pR * g.gamma * rcp2(rR)));
   const f2 SL = min2(uL, uR) - cmax;
   const f2 SR = max2(uL, uR) + cmax;
   const f2 rcL = rL * (uL - SL);
@@ -136,23 +136,23 @@ __device__ __forceinline__ void hllc(const Q2 &qL, const Q2 &qR, Q2 &f, f2 &pout
   const f2 rd = rcp2(rcR + rcL);
   const f2 uS = (fma2(rcR, uR, rcL * uL) + (pL - pR)) * rd;
   const f2 pS = fma2(rcL * rcR, uL - uR, fma2(rcR, pL, rcL * pR)) * rd;
-  const b2 sideL = gt0(uS);
-  const f2 rK = sel2(sideL, rL, rR);
-  const f2 uK = sel2(sideL, uL, uR);
-  const f2 pK = sel2(sideL, pL, pR);
-  const f2 EK = sel2(sideL, EL, ER);
-  const f2 SK = sel2(sideL, SL, SR);
+  const b2 bL = gt0(SL), sR = gt0(SR), sideL = gt0(uS);
+  const b2 left{bL.x || sideL.x, bL.y || sideL.y};
+  const b2 star{!bL.x && (sideL.x || sR.x), !bL.y && (sideL.y || sR.y)};
+  const f2 rK = sel2(left, rL, rR);
+  const f2 uK = sel2(left, uL, uR);
+  const f2 sv = sel2(left, vL, vR);
+  const f2 pK = sel2(left, pL, pR);
+  const f2 SK = sel2(left, SL, SR);
+  const f2 EK = fma2(g.half * rK, fma2(uK, uK, sv * sv), pK * g.entho);
   const f2 rd2 = rcp2(SK - uS);
   const f2 SKu = SK - uK;
   const f2 rS = (rK * SKu) * rd2;
   const f2 ES = fma2(pS, uS, SKu * EK - pK * uK) * rd2;
-  const b2 bL = gt0(SL), sR = gt0(SR);
-  const b2 bS{!bL.x && (sideL.x || sR.x), !bL.y && (sideL.y || sR.y)};
-  const f2 sr = sel2(bL, rL, sel2(bS, rS, rR));
-  const f2 su = sel2(bL, uL, sel2(bS, uS, uR));
-  const f2 sv = sel2(bL, vL, sel2(bS, sel2(sideL, vL, vR), vR));
-  const f2 sp = sel2(bL, pL, sel2(bS, pS, pR));
-  const f2 E = sel2(bL, EL, sel2(bS, ES, ER));
+  const f2 sr = sel2(star, rS, rK);
+  const f2 su = sel2(star, uS, uK);
+  const f2 sp = sel2(star, pS, pK);
+  const f2 E = sel2(star, ES, EK);
   pout = sp;
   f.r = sr * su;
   f.u = fma2(f.r, su, sp);
@@ -170,12 +170,13 @@ __device__ __forceinline__ Q2 solve(const Q2 &qL, const Q2 &qR, const Gas2 &g, f
   return f;
 }
 
-// pressure_of for the pair (batch_common.cuh); the low-Mach recovery per column
-__device__ __forceinline__ f2 pressure2(f2 dE, float bg_e, f2 r, f2 u, f2 v, float gm1, int lowmach) {
-  if (lowmach)
-    return make_float2(pressure_of(dE.x, bg_e, r.x, u.x, v.x, gm1, 1), pressure_of(dE.y, bg_e, r.y, u.y, v.y, gm1, 1));
+// pressure_of for the pair (batch_common.cuh), and its low-Mach recovery per column
+__device__ __forceinline__ f2 pressure2(f2 dE, float bg_e, f2 r, f2 u, f2 v, float gm1) {
   const f2 ek = (F2(0.5f) * r) * fma2(u, u, v * v);
   return ((dE - ek) + F2(bg_e)) * F2(gm1);
+}
+__device__ __forceinline__ f2 pressure2_lowmach(f2 dE, float bg_e, f2 r, f2 u, f2 v, float gm1) {
+  return make_float2(pressure_of(dE.x, bg_e, r.x, u.x, v.x, gm1, 1), pressure_of(dE.y, bg_e, r.y, u.y, v.y, gm1, 1));
 }
 
 // consToPrim of a stored offset pair (States.h:32-43) with the negative reset
@@ -184,12 +185,15 @@ __device__ __forceinline__ Q2 to_prim(const f2 u[4], const SimView &S) {
   f2 r = u[0] + F2(S.bg_r);
   const f2 rr = rcp2(r);
   const f2 uu = u[1] * rr, vv = u[2] * rr;
-  f2 p = pressure2(u[3], S.bg_e, r, uu, vv, S.gm1, S.lowmach);
-  if (!S.avg) {
-    if (r.x < 0.f) r.x = 1e-8f;
-    if (r.y < 0.f) r.y = 1e-8f;
-    if (p.x < 0.f) p.x = 1e-8f;
-    if (p.y < 0.f) p.y = 1e-8f;
+  f2 p = pressure2(u[3], S.bg_e, r, uu, vv, S.gm1);
+  if (S.lowmach || fminf(fminf(r.x, r.y), fminf(p.x, p.y)) < 0.f) {
+    if (S.lowmach) p = pressure2_lowmach(u[3], S.bg_e, r, uu, vv, S.gm1);
+    if (!S.avg) {
+      if (r.x < 0.f) r.x = 1e-8f;
+      if (r.y < 0.f) r.y = 1e-8f;
+      if (p.x < 0.f) p.x = 1e-8f;
+      if (p.y < 0.f) p.y = 1e-8f;
+    }
   }
   return Q2{r, uu, vv, p};
 }
@@ -237,7 +241,9 @@ __device__ __forceinline__ void march2_item(const BatchArgs &a, const WorkItem i
   const int ntiles = FV2D_SIM(W, ntx) * FV2D_SIM(W, nty);
   const int Nx = S.Nx, Ny = S.Ny;
   const int gxl = item.tx * STRIP + 2 * lane;  // padded column of the pair's first half (even)
-  const bool colok = gxl < Nx + 4;             // then gxl + 1 < pitch: the pair lies in the row
+  // the pair a lane loads: its own (gxl + 1 < pitch: it lies in the row), or,
+  // past the row's end, its last one, which never reaches an output column
+  const int gld = min(gxl, (Nx + 3) & ~1);
   const bool out0 = lane >= 1 && lane < 31 && gxl - 2 < Nx;  // columns 2..61 of the strip are interior
   const bool out1 = out0 && gxl - 1 < Nx;
   const int band = FV2D_SIM(W, band);
@@ -245,13 +251,9 @@ __device__ __forceinline__ void march2_item(const BatchArgs &a, const WorkItem i
   const f2 dtdx = F2(S.dt * S.inv_dx), dtdy = F2(S.dt * S.inv_dy);
 
   auto load = [&](int L, f2 u[4]) {  // padded row L, columns gxl and gxl + 1
-    const long long g = (long long)L * S.P + gxl;
-    if (colok) {
+    const long long g = (long long)L * S.P + gld;
 #pragma unroll
-      for (int k = 0; k < 4; ++k) u[k] = __ldg(reinterpret_cast<const float2 *>(S.src + k * S.PL + g));
-    } else {
-      u[0] = F2(1.f); u[1] = F2(0.f); u[2] = F2(0.f); u[3] = F2(1.f);  // never reaches an output column
-    }
+    for (int k = 0; k < 4; ++k) u[k] = __ldg(reinterpret_cast<const float2 *>(S.src + k * S.PL + g));
   };
   const Q2 z = zero();
   auto yslope = [&](const Q2 &dl, const Q2 &dr) {
@@ -277,6 +279,8 @@ __device__ __forceinline__ void march2_item(const BatchArgs &a, const WorkItem i
   // The row loop of batch_march.cuh, with its four window-fill iterations
   // peeled into a prologue so that the main loop's y-face and x-face solves,
   // which are independent, share one block the compiler can interleave.
+  // The prologue's rows are loaded together: row by row, each of its short
+  // iterations waited for memory (KH 512^2 1.52 against 1.45 ms per 100 steps).
   // Iteration L loads padded row L and (from L = j0 + 4 on) updates row
   // C = L - 2.  Both copies of the row entry and of the y face are the same
   // functions of the same operands, and every operation in them is an explicit
@@ -284,11 +288,14 @@ __device__ __forceinline__ void march2_item(const BatchArgs &a, const WorkItem i
   // to contract), so a face that two bands share gets bit-identical fluxes from
   // the prologue of one and the main loop of the other: the step stays exactly
   // conservative.
+  // The loop is bound by instruction issue and by the latency of its chain at 16
+  // warps per SM, so rare work (negative or NaN cells, the low-Mach recovery)
+  // leaves it through one branch at each end: KH 2048^2, PLM + HLLC, 49.0 G
+  // cell-updates/s with a select for each case, 56.3 G now.
   // The window carries the primitives of rows L - 2 and L - 1 (q0, qp), the
   // y slope of row L - 2, the y flux of face C - 1/2 and the prefetched next
   // row; the conservative row C is read again at its update (an L1 hit: it
-  // was loaded two iterations earlier) and the primitives of row C - 1 are
-  // rebuilt from memory only when conduction or viscosity need them.
+  // was loaded two iterations earlier).
   Q2 q0 = z, qp = z, h0 = z, Gm = z;
   f2 Unext[4];
   float lmax = 0.f;
@@ -303,13 +310,71 @@ __device__ __forceinline__ void march2_item(const BatchArgs &a, const WorkItem i
     f2 pout;
     return swap_uv(solve<RS>(swap_uv(face(q0, h0, hp5)), swap_uv(face(qp, hp, hm5)), gas, pout));
   };
-  load(j0, Unext);
-  for (int L = j0; L < j0 + 4; ++L) {  // jend >= j0 + 1: row L + 1 is in the band's window
-    const f2 Un[4] = {Unext[0], Unext[1], Unext[2], Unext[3]};
-    load(L + 1, Unext);
+  // Conduction (constant conductivity, ThermalConduction.h:36-73) and viscosity
+  // (Viscosity.h:27-119): a face's heat flux and viscous terms are formed once,
+  // those of an x face in the column on its right, those of a y face when the
+  // march crosses it, as the cells of a face share them in the reference up to
+  // the sign.  The window carries the temperature, the x span of the velocities
+  // and the y face terms of row C, and row C - 1's velocities: half the
+  // arithmetic, a third of the shuffles and none of the loads and conversions of
+  // forming the four faces of each cell from its 3 x 3 neighbours (RT 1024 x
+  // 3072, HLL, ms per 100 steps: 9.38 | 8.6; the one-column march 8.9).
+  struct V2 {
+    f2 u, v;
+  };
+  struct T2 {
+    f2 u, v, e;
+  };
+  f2 T0 = F2(0.f), Hm = F2(0.f);
+  V2 E0{F2(0.f), F2(0.f)}, um = E0;
+  T2 Ym{F2(0.f), F2(0.f), F2(0.f)};
+  auto temperature = [&](const Q2 &q) { return q.p * rcp2(q.r); };
+  auto yheat = [&](f2 Ta, f2 Tb) { return F2(S.kappa * S.inv_dy) * (Tb - Ta); };
+  auto xspan = [&](const Q2 &q) { return V2{right(q.u) - left(q.u), right(q.v) - left(q.v)}; };
+  // mu times (tau_nn, tau_nt, tau . velocity) of a face from the velocities'
+  // normal and transverse derivatives and their means
+  auto stress = [&](f2 dndn, f2 dtdn, f2 dndt, f2 dtdt, f2 qn, f2 qt) {
+    const f2 tnn = F2(4.f / 3.f) * dndn - F2(2.f / 3.f) * dtdt, tnt = dtdn + dndt;
+    const f2 mu = F2(S.mu);
+    return T2{mu * tnn, mu * tnt, mu * fma2(tnn, qn, tnt * qt)};
+  };
+  auto yvisc = [&](const V2 &Ea, const V2 &Eb) {  // between q0's row and qp's
+    const f2 d = F2(S.inv_dy), c = F2(0.25f * S.inv_dx);
+    const T2 t = stress(d * (qp.v - q0.v), d * (qp.u - q0.u), c * (Eb.v + Ea.v), c * (Eb.u + Ea.u), hp5 * (qp.v + q0.v),
+                        hp5 * (qp.u + q0.u));
+    return T2{t.v, t.u, t.e};
+  };
+  auto xvisc = [&]() {  // between the columns of q0's row
+    const f2 d = F2(S.inv_dx), c = F2(0.25f * S.inv_dy);
+    const V2 D{qp.u - um.u, qp.v - um.v}, Dw{left(D.u), left(D.v)};
+    const f2 uw = left(q0.u), vw = left(q0.v);
+    return stress(d * (q0.u - uw), d * (q0.v - vw), c * (D.u + Dw.u), c * (D.v + Dw.v), hp5 * (q0.u + uw),
+                  hp5 * (q0.v + vw));
+  };
+  // jend >= j0 + 1: rows j0 to j0 + 4 are in the band's window
+  f2 Ufill[4][4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) load(j0 + k, Ufill[k]);
+  load(j0 + 4, Unext);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int L = j0 + k;
     Q2 qn, hp;
-    enter(Un, qn, hp);
+    enter(Ufill[k], qn, hp);
     if (L == j0 + 3) Gm = yface(hp);
+    if constexpr (TCV) {  // row j0 + 1's, then those of the face below it
+      if (L >= j0 + 2 && S.tc) {
+        const f2 Tp = temperature(qp);
+        Hm = yheat(T0, Tp);
+        T0 = Tp;
+      }
+      if (L >= j0 + 2 && S.visc) {
+        const V2 Ep = xspan(qp);
+        Ym = yvisc(E0, Ep);
+        E0 = Ep;
+        um = V2{q0.u, q0.v};
+      }
+    }
     q0 = qp;
     qp = qn;
     h0 = hp;
@@ -317,6 +382,8 @@ __device__ __forceinline__ void march2_item(const BatchArgs &a, const WorkItem i
   for (int L = j0 + 4; L < jend + 4; ++L) {
     const int C = L - 2;
     const int j = C - 2;
+    f2 U0[4];
+    load(C, U0);
     const f2 Un[4] = {Unext[0], Unext[1], Unext[2], Unext[3]};
     if (L + 1 < jend + 4) load(L + 1, Unext);
     Q2 qn, hp;
@@ -331,8 +398,7 @@ __device__ __forceinline__ void march2_item(const BatchArgs &a, const WorkItem i
 
       // update in the reference's order: x flux, x gravity, y flux, y
       // gravity, conduction, viscosity (Update.h:114-168, 176-191)
-      f2 un[4], U0[4];
-      load(C, U0);
+      f2 un[4];
       un[0] = fma2(Fw.r - Fe.r, dtdx, U0[0]);
       un[1] = fma2(Fw.u - Fe.u, dtdx, U0[1]);
       un[2] = fma2(Fw.v - Fe.v, dtdx, U0[2]);
@@ -350,67 +416,29 @@ __device__ __forceinline__ void march2_item(const BatchArgs &a, const WorkItem i
         un[2] = fma2(dt2 * q0.r, F2(S.gy), un[2]);
         un[3] = fma2(dt2 * (hp5 * (Gm.r + Gp.r)), F2(S.gy), un[3]);
       }
-      Q2 qm = z;  // primitives of row C - 1
-      if (TCV && (S.tc || S.visc)) {
-        f2 Um[4];
-        load(C - 1, Um);
-        qm = to_prim(Um, S);
-      }
-      if (TCV && S.tc) {  // constant conductivity (ThermalConduction.h:36-73)
-        const f2 TC = q0.p * rcp2(q0.r);
-        const f2 TL = left(TC), TR = right(TC);
-        const f2 TU = qm.p * rcp2(qm.r), TD = qp.p * rcp2(qp.r);
-        const f2 kx = F2(S.kappa * S.inv_dx), ky = F2(S.kappa * S.inv_dy);
-        const f2 FL = kx * (TC - TL), FR = kx * (TR - TC);
-        const f2 FU = ky * (TC - TU), FD = ky * (TD - TC);
-        un[3] = un[3] + fma2(dtdx, FR - FL, dtdy * (FD - FU));
-      }
-      if (TCV && S.visc) {
-        // 3x3 stencil of velocities: rows C-1, C, C+1 (qm, q0, qp) x columns -1, 0, +1
-        const f2 odx = F2(S.inv_dx), ody = F2(S.inv_dy);
-        f2 u_[3][3], v_[3][3];
-        const Q2 *rws[3] = {&qm, &q0, &qp};
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-          u_[r][1] = rws[r]->u;
-          v_[r][1] = rws[r]->v;
-          u_[r][0] = left(u_[r][1]);
-          v_[r][0] = left(v_[r][1]);
-          u_[r][2] = right(u_[r][1]);
-          v_[r][2] = right(v_[r][1]);
+      if constexpr (TCV) {
+        if (S.tc) {
+          const f2 Tp = temperature(qp);
+          const f2 Hp = yheat(T0, Tp);
+          const f2 Hw = F2(S.kappa * S.inv_dx) * (T0 - left(T0));  // x faces as above: the pair's west ones
+          un[3] = un[3] + fma2(dtdx, right(Hw) - Hw, dtdy * (Hp - Hm));
+          T0 = Tp;
+          Hm = Hp;
         }
-        auto U_ = [&](int dj, int di) { return u_[dj + 1][di + 1]; };
-        auto V_ = [&](int dj, int di) { return v_[dj + 1][di + 1]; };
-        const f2 c43 = F2(4.f / 3.f), c23 = F2(2.f / 3.f), q25 = F2(0.25f);
-        f2 f1 = F2(0.f), f2_ = F2(0.f), f3 = F2(0.f);
-#pragma unroll
-        for (int side = 1; side < 3; ++side) {
-          const f2 smu = F2(side == 1 ? -S.mu : S.mu);
-          const int s = side - 1, sm1 = side - 2;
-          {
-            const f2 qiu = (U_(0, s) + U_(0, sm1)) * hp5, qiv = (V_(0, s) + V_(0, sm1)) * hp5;
-            const f2 dudx = odx * (U_(0, s) - U_(0, sm1)), dvdx = odx * (V_(0, s) - V_(0, sm1));
-            const f2 dudy = (q25 * ody) * ((U_(1, s) - U_(-1, s)) + (U_(1, sm1) - U_(-1, sm1)));
-            const f2 dvdy = (q25 * ody) * ((V_(1, s) - V_(-1, s)) + (V_(1, sm1) - V_(-1, sm1)));
-            const f2 txx = c43 * dudx - c23 * dvdy, txy = dvdx + dudy;
-            f1 = fma2(smu, txx, f1);
-            f2_ = fma2(smu, txy, f2_);
-            f3 = fma2(smu, fma2(txx, qiu, txy * qiv), f3);
-          }
-          {
-            const f2 qiu = (U_(s, 0) + U_(sm1, 0)) * hp5, qiv = (V_(s, 0) + V_(sm1, 0)) * hp5;
-            const f2 dudy = ody * (U_(s, 0) - U_(sm1, 0)), dvdy = ody * (V_(s, 0) - V_(sm1, 0));
-            const f2 dudx = (q25 * odx) * ((U_(s, 1) - U_(s, -1)) + (U_(sm1, 1) - U_(sm1, -1)));
-            const f2 dvdx = (q25 * odx) * ((V_(s, 1) - V_(s, -1)) + (V_(sm1, 1) - V_(sm1, -1)));
-            const f2 tyy = c43 * dvdy - c23 * dudx, txy = dvdx + dudy;
-            f1 = fma2(smu, txy, f1);
-            f2_ = fma2(smu, tyy, f2_);
-            f3 = fma2(smu, fma2(txy, qiu, tyy * qiv), f3);
-          }
+        if (S.visc) {
+          const V2 Ep = xspan(qp);
+          const T2 Yp = yvisc(E0, Ep);
+          const T2 Xw = xvisc();
+          const f2 f1 = (right(Xw.u) - Xw.u) + (Yp.u - Ym.u);
+          const f2 f2_ = (right(Xw.v) - Xw.v) + (Yp.v - Ym.v);
+          const f2 f3 = (right(Xw.e) - Xw.e) + (Yp.e - Ym.e);
+          un[1] = fma2(f1, dt2, un[1]);
+          un[2] = fma2(f2_, dt2, un[2]);
+          un[3] = fma2(f3, dt2, un[3]);
+          E0 = Ep;
+          Ym = Yp;
+          um = V2{q0.u, q0.v};
         }
-        un[1] = fma2(f1, dt2, un[1]);
-        un[2] = fma2(f2_, dt2, un[2]);
-        un[3] = fma2(f3, dt2, un[3]);
       }
 
       if (out0) {
@@ -432,27 +460,32 @@ __device__ __forceinline__ void march2_item(const BatchArgs &a, const WorkItem i
             d[0] = un[k].x;
         }
         if (S.last) {
-          // primitive state of the new cells for the next dt, negative guard
-          f2 r = un[0] + F2(S.bg_r);
+          // primitive state of the new cells for the next dt; the negative
+          // and NaN guards leave the common path through one test
+          const f2 r = un[0] + F2(S.bg_r);
           const f2 rr = rcp2(r);
           const f2 u = un[1] * rr, v = un[2] * rr;
-          f2 p = pressure2(un[3], S.bg_e, r, u, v, S.gm1, S.lowmach);
-          const float rx[2] = {r.x, r.y}, ux[2] = {u.x, u.y}, vx[2] = {v.x, v.y}, px[2] = {p.x, p.y};
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            if (h == 1 && !out1) break;
-            float rh = rx[h], ph = px[h];
-            nnan += is_nan_f(rh) | is_nan_f(ux[h]) | is_nan_f(vx[h]) | is_nan_f(ph);
-            nneg += (rh < 0.f) + (ph < 0.f);
-            if (rh < 0.f) rh = 1e-8f;
-            if (ph < 0.f) ph = 1e-8f;
-            const float cs = sqrtf(ph * S.gamma * __fdividef(1.f, rh));
-            const float ih = (cs + fabsf(ux[h])) * S.inv_dx + (cs + fabsf(vx[h])) * S.inv_dy;
-            if (ih > lmax) lmax = ih;  // NaN never enters
+          f2 p = pressure2(un[3], S.bg_e, r, u, v, S.gm1);
+          f2 cs2 = p * F2(S.gamma) * rr;
+          // a NaN of any field reaches the pressure
+          if (S.lowmach || !(min_nan(min_nan(r.x, p.x), min_nan(r.y, p.y)) >= 0.f)) {
+            if (S.lowmach) p = pressure2_lowmach(un[3], S.bg_e, r, u, v, S.gm1);
+            auto guard = [&](float rh, float ph, float rrh, float &c2) {
+              nnan += is_nan_f(ph);
+              nneg += (rh < 0.f) + (ph < 0.f);
+              c2 = (ph < 0.f ? 1e-8f : ph) * S.gamma * (rh < 0.f ? __fdividef(1.f, 1e-8f) : rrh);
+            };
+            guard(r.x, p.x, rr.x, cs2.x);
+            if (out1) guard(r.y, p.y, rr.y, cs2.y);
           }
+          const f2 cs = sqrt2(cs2);
+          const f2 cu = make_float2(cs.x + fabsf(u.x), cs.y + fabsf(u.y));
+          const f2 cv = make_float2(cs.x + fabsf(v.x), cs.y + fabsf(v.y));
+          const f2 ih = fma2(cu, F2(S.inv_dx), cv * F2(S.inv_dy));
+          lmax = fmaxf(lmax, fmaxf(ih.x, out1 ? ih.y : 0.f));  // NaN never enters
         } else {
-          nnan += is_nan_f(un[0].x) | is_nan_f(un[1].x) | is_nan_f(un[2].x) | is_nan_f(un[3].x);
-          if (out1) nnan += is_nan_f(un[0].y) | is_nan_f(un[1].y) | is_nan_f(un[2].y) | is_nan_f(un[3].y);
+          nnan += is_nan_f(min_nan(min_nan(un[0].x, un[1].x), min_nan(un[2].x, un[3].x)));
+          if (out1) nnan += is_nan_f(min_nan(min_nan(un[0].y, un[1].y), min_nan(un[2].y, un[3].y)));
         }
         // ghost copies (BoundaryConditions.h:82-147, inverse map), per column
         const int i0 = gxl - 2;
