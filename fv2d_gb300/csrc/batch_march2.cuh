@@ -246,6 +246,7 @@ __device__ __forceinline__ void march2_item(const BatchArgs &a, const WorkItem i
   const int gld = min(gxl, (Nx + 3) & ~1);
   const bool out0 = lane >= 1 && lane < 31 && gxl - 2 < Nx;  // columns 2..61 of the strip are interior
   const bool out1 = out0 && gxl - 1 < Nx;
+  const bm::XGhosts xg = out0 ? bm::x_ghosts(gxl - 2, out1, Nx, S.bcx) : bm::XGhosts{0u};
   const int band = FV2D_SIM(W, band);
   const int j0 = item.ty * band, jend = min(j0 + band, Ny);
   const f2 dtdx = F2(S.dt * S.inv_dx), dtdy = F2(S.dt * S.inv_dy);
@@ -487,33 +488,31 @@ __device__ __forceinline__ void march2_item(const BatchArgs &a, const WorkItem i
           nnan += is_nan_f(min_nan(min_nan(un[0].x, un[1].x), min_nan(un[2].x, un[3].x)));
           if (out1) nnan += is_nan_f(min_nan(min_nan(un[0].y, un[1].y), min_nan(un[2].y, un[3].y)));
         }
-        // ghost copies (BoundaryConditions.h:82-147, inverse map), per column
-        const int i0 = gxl - 2;
-        const bool ey = (j < 2 || j >= Ny - 2);
-        const bool ex = (i0 < 2 || i0 + 1 >= Nx - 2);
-        if (ex || ey) {
-          const float ur[2] = {un[0].x, un[0].y}, uu[2] = {un[1].x, un[1].y}, uv[2] = {un[2].x, un[2].y},
-                      ue[2] = {un[3].x, un[3].y};
-          for (int h = 0; h < 2; ++h) {
-            if (h == 1 && !out1) break;
-            const int i = i0 + h;
-            const bool exh = (i < 2 || i >= Nx - 2);
-            if (!exh && !ey) continue;
-            int tx[5], ty[5];
-            bool nx[5], ny[5];
-            tx[0] = i; nx[0] = false;
-            ty[0] = j; ny[0] = false;
-            const int cx = 1 + (exh ? ghost_targets(i, Nx, S.bcx, tx + 1, nx + 1) : 0);
-            const int cy = 1 + (ey ? ghost_targets(j, Ny, S.bcy, ty + 1, ny + 1) : 0);
-            for (int b = 0; b < cy; ++b)
-              for (int c = 0; c < cx; ++c) {
-                if (b == 0 && c == 0) continue;
-                const long long gg = (long long)(ty[b] + 2) * S.P + (tx[c] + 2);
-                S.dst[gg] = ur[h];
-                S.dst[S.PL + gg] = nx[c] ? -uu[h] : uu[h];
-                S.dst[2 * S.PL + gg] = ny[b] ? -uv[h] : uv[h];
-                S.dst[3 * S.PL + gg] = ue[h];
+        // ghost copies (BoundaryConditions.h:82-147, inverse map): the pair's
+        // row, then, for rows whose ghosts copy it, each of those rows
+        const bool ey = j < 2 || j >= Ny - 2;
+        if (ey || xg.any()) {
+#pragma unroll 1
+          for (int t = ey ? 0 : 4; t < 5; ++t) {
+            int ty = j;
+            bool flip = false;
+            if (t < 4) {
+              ty = t < 2 ? t - 2 : Ny + t - 2;
+              if (ghost_source(ty, Ny, S.bcy, &flip) != j) continue;
+            }
+            float *row = S.dst + (long long)(ty + 2) * S.P;
+#pragma unroll
+            for (int k = 0; k < 4; ++k, row += S.PL) {
+              f2 x = un[k];
+              if (k == 2 && flip) x = make_float2(-x.x, -x.y);
+              if (t < 4) {
+                if (out1) *reinterpret_cast<float2 *>(row + gxl) = x;
+                else row[gxl] = x.x;
               }
+              if (k == 1 && S.bcx == 1) x = make_float2(-x.x, -x.y);  // reflecting
+              if (xg.any()) row[xg.a()] = xg.ha() ? x.y : x.x;
+              if (xg.two()) row[xg.b()] = xg.hb() ? x.y : x.x;
+            }
           }
         }
       }

@@ -68,3 +68,44 @@ def test_nan_cells_fail_their_request(gpu_lib, config, stepping, diffusive):
         res = {r.id: r for r in s.poll()}
         assert res[b].status == ERR_NUMERIC and res[b].steps < 20
         assert res[g].status == 0 and res[g].steps == 20
+
+
+@pytest.mark.parametrize("scheme", ["plain", "diffusive", "extended"])
+@pytest.mark.parametrize("bcx", ["BC_ABSORBING", "BC_REFLECTING", "BC_PERIODIC"])
+def test_ghost_columns_of_any_width(gpu_lib, scheme, bcx):
+    """The ghost cells that the march kernels write, at widths around their
+    strips (28 and 60 columns) and at the narrowest grid, against the binary64
+    path.  A step rounds each of its ~50 chained operations to 2^-24 of the
+    fields' scale, so 8 steps stay below 8 * 50 * 6e-8 = 2.4e-5 of it; a wrong
+    ghost is an error of order 0.01 in the cells beside it."""
+    import numpy as np
+    import fv2d_gb300 as fv
+    from fv2d_gb300.serve import Server
+    f = fv.as_float32
+    extra = {"plain": {}, "diffusive": dict(thermal_conductivity_active=1, kappa=f(1e-4), viscosity_active=1,
+                                            mu=f(1e-4)),
+             "extended": dict(reconstruction=fv.MUSCL_HANCOCK)}[scheme]
+    configs = {"plain": ["28/32x20/march", "60/32x16/march2"],
+               "diffusive": ["28/32x20/march", "60/32x16/march2-diff"], "extended": [None]}[scheme]
+    runs = []
+    for nx in (16, 17, 27, 28, 29, 59, 60, 61, 62, 120, 121):
+        for bcy, ny, ts in ((fv.BC_REFLECTING, 16, fv.TS_EULER), (fv.BC_PERIODIC, 19, fv.TS_RK2),
+                            (fv.BC_ABSORBING, 21, fv.TS_EULER)):
+            p = dict(Nx=nx, Ny=ny, gamma0=f(1.4), CFL=f(0.4), reconstruction=fv.PLM, riemann_solver=fv.HLLC,
+                     boundary_x=getattr(fv, bcx), boundary_y=bcy, time_stepping=ts, seed=nx)
+            p.update(extra)
+            runs.append(fv.default_params(**p))
+    for config in configs:
+        with Server(budget_bytes=1e9, autotune=False, tile_config=config) as s:
+            ids = [s.submit("kh_step", p, 8) for p in runs]
+            assert s.drain(120) == 0
+            res = {r.id: r for r in s.poll()}
+            for p, i in zip(runs, ids):
+                assert res[i].status == 0
+                sim = fv.Simulation(p)
+                sim.init_problem("kh_step")
+                sim.advance(8, 1e30)
+                want, got = np.asarray(sim.get_prim()), np.asarray(s.get_prim(i), dtype=float)
+                scale = np.abs(want).max(axis=(0, 1))
+                scale[1:3] = scale[1:3].max()
+                assert (np.abs(got - want).max(axis=(0, 1)) <= 2.4e-5 * scale).all(), (config, p.Nx, p.Ny)
