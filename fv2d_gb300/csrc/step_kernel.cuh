@@ -218,11 +218,29 @@ __device__ __forceinline__ T load_words(const T *p) {
   return v;
 }
 
-template <class T_, int RECON, int RS, bool VISC>
-__global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
+// What a step is compiled for: an Euler step of the conservation laws alone; with
+// the RK2 stages, gravity, the well-balanced boundary flux and conduction, decided
+// as it runs; with viscosity as well (it takes shared memory and registers).  The
+// tests of the second form cut the update into blocks that the compiler schedules
+// one by one: HLLC, ms per 8 steps of 2048^2, PLM 8.33 | 8.13 without them, PCM
+// 6.35 | 6.17, MUSCL-Hancock 12.8 | 12.3, Sod 512 x 8 15.7 | 15.3 us a step.  PLM with
+// HLL runs 1.7 % slower without them on full grids (11.31 | 11.51) and keeps them.
+enum StepForm { FORM_PLAIN = 0, FORM_SOURCES = 1, FORM_VISCOUS = 2 };
+
+template <class T_, int RECON, int RS>
+constexpr bool has_plain_form() {
+  return T_::TX < 16 || RS != RS_HLL || RECON != RECON_PLM;
+}
+
+template <class T_, int RECON, int RS, int FORM>
+__global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(FORM == FORM_VISCOUS))
     step_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant__ CUtensorMap tmQ1,
                 const StepArgs a) {
+  constexpr bool VISC = FORM == FORM_VISCOUS;
   using L = Smem<T_, RECON, VISC>;
+  const bool has_tc = FORM != FORM_PLAIN && a.tc, has_wb = FORM != FORM_PLAIN && a.wb;
+  const int grav_mode = FORM != FORM_PLAIN ? a.grav_mode : 0;
+  const int stage = FORM != FORM_PLAIN ? a.stage : STAGE_EULER;
   constexpr int TX = T_::TX, TY = T_::TY, SW = T_::SW, SH = T_::SH, NT = T_::NT;
   constexpr int SOFT = step_soft_mul<T_, RS>(VISC);
   // Aligned by offsetting the shared array itself (not through an integer
@@ -254,12 +272,12 @@ __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
   if (tid == 0) {
     mbar_init(&mbar, 1);
     fence_mbar_init();
-    const bool corrects = a.stage == STAGE_RK2_CORRECT;
+    const bool corrects = stage == STAGE_RK2_CORRECT;
     // of a chained sequence, the corrector's clock is the one its predictor stored
     const int from = !a.chained ? 0 : (a.step + corrects) & 1;
     Clock c = load_words(&st->clock[from]);
     const bool commits = a.chained && a.step > 0 && !corrects && c.status == RUN_RUNNING;
-    const int par = commits && a.stage == STAGE_EULER ? 1 - c.parity : c.parity;
+    const int par = commits && stage == STAGE_EULER ? 1 - c.parity : c.parity;
     const int src = corrects ? 1 - par : par;
     // the load needs the parity alone: the rest of the clock is formed behind it
     mbar_expect_tx(&mbar, 4u * SH * SW * sizeof(double));
@@ -283,7 +301,7 @@ __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
     return;
   }
   const double dt = now.dt;
-  const int dst = (a.stage == STAGE_RK2_CORRECT) ? now.parity : 1 - now.parity;
+  const int dst = (stage == STAGE_RK2_CORRECT) ? now.parity : 1 - now.parity;
   StepSums *pending = &st->pending[a.chained ? a.step & 3 : 0];
   mbar_wait_bounded(&mbar, &st->error);
 
@@ -352,7 +370,7 @@ __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
       }
     }
   }
-  if (a.tc) {
+  if (has_tc) {
     for (int it = tid; it < L::R1; it += NT) {
       const int ly = it / L::R1W + 1, lx = it % L::R1W + 1;
       if (ly > ny + 2 || lx > nx + 2) continue;  // past the grid's ghost ring
@@ -496,9 +514,9 @@ __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
   // ---- 4./5. cell update, conversion, stores, reductions -------------------
   double lmax = -1.0;
   unsigned cnt_rho = 0, cnt_prs = 0, cnt_nan = 0;
-  const bool final_stage = (a.stage != STAGE_RK2_PREDICT);
-  const double *Usrc = (a.stage == STAGE_RK2_CORRECT) ? a.U1 : a.U;
-  double *Udst = (a.stage == STAGE_RK2_PREDICT) ? a.U1 : a.U;
+  const bool final_stage = (stage != STAGE_RK2_PREDICT);
+  const double *Usrc = (stage == STAGE_RK2_CORRECT) ? a.U1 : a.U;
+  double *Udst = (stage == STAGE_RK2_PREDICT) ? a.U1 : a.U;
   double *Qd = a.Q[dst];
   const long long PL = a.plane;
   const int P = a.pitch;
@@ -548,8 +566,8 @@ __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
         un[k] = add(un[k], ddivc(d0, a.dx, a.inv_dx, a.dx_pow2, a.rw_dx));
         un[k + 1] = add(un[k + 1], ddivc(d1, a.dx, a.inv_dx, a.dx_pow2, a.rw_dx));
       }
-      if (a.grav_mode) {
-        const double gv = (a.grav_mode == 1) ? a.gxf : (double)a.grav_row[j];
+      if (grav_mode) {
+        const double gv = (grav_mode == 1) ? a.gxf : (double)a.grav_row[j];
         gravity(un, rho, FL0, FR0, gv);
       }
     }
@@ -564,9 +582,9 @@ __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
         FR[k] = SMI(F + k * S + TX);
       }
       double gv = 0.0;
-      if (a.grav_mode) gv = (a.grav_mode == 1) ? a.gyf : (double)a.grav_row[j];
-      if (a.wb && (j == 0 || j == a.Ny - 1)) {  // Update.h:149-156
-        const double gy = (a.grav_mode == 0) ? 0.0 : gv;
+      if (grav_mode) gv = (grav_mode == 1) ? a.gyf : (double)a.grav_row[j];
+      if (has_wb && (j == 0 || j == a.Ny - 1)) {  // Update.h:149-156
+        const double gy = (grav_mode == 0) ? 0.0 : gv;
         if (j == 0) {
           const double poutR = SMI(L::PY + (ry + 1) * TX + rx);
           FL[0] = 0.0; FL[1] = 0.0; FL[2] = poutR - rho * gy * a.dy; FL[3] = 0.0;
@@ -582,10 +600,10 @@ __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
         un[k] = add(un[k], ddivc(d0, a.dy, a.inv_dy, a.dy_pow2, a.rw_dy));
         un[k + 1] = add(un[k + 1], ddivc(d1, a.dy, a.inv_dy, a.dy_pow2, a.rw_dy));
       }
-      if (a.grav_mode) gravity(un, rho, FL[0], FR[0], gv);
+      if (grav_mode) gravity(un, rho, FL[0], FR[0], gv);
     }
     // thermal conduction (ThermalConduction.h:46-106)
-    if (a.tc) {
+    if (has_tc) {
       const double TC = sR1(L::T, 0, ly, lx);
       const double TL = sR1(L::T, 0, ly, lx - 1), TR = sR1(L::T, 0, ly, lx + 1);
       const double TU = sR1(L::T, 0, ly - 1, lx), TD = sR1(L::T, 0, ly + 1, lx);
@@ -639,7 +657,7 @@ __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
       un[3] = add(un[3], mulx<12, SOFT>(add(fx3, fy3), dt));
     }
     // RK2 corrector: 0.5 * (U0 + Unew) (Update.h:214-220)
-    if (a.stage == STAGE_RK2_CORRECT) {
+    if (stage == STAGE_RK2_CORRECT) {
 #pragma unroll
       for (int k = 0; k < 4; ++k) un[k] = fv_half(add(a.U[k * PL + g], un[k]));
     }
@@ -674,22 +692,54 @@ __global__ void __launch_bounds__(T_::NT, step_ctas_per_sm<T_, RECON, RS>(VISC))
     // ghost cells that copy this cell (BoundaryConditions.h:82-147)
     const bool ex = (i < 2 || i >= a.Nx - 2), ey = (j < 2 || j >= a.Ny - 2);
     if (ex || ey) {
-      int tx[5], ty[5];
-      bool fx[5], fy[5];
-      tx[0] = i; fx[0] = false;
-      ty[0] = j; fy[0] = false;
-      const int cx = 1 + (ex ? ghost_targets(i, a.Nx, a.bcx, tx + 1, fx + 1) : 0);
-      const int cy = 1 + (ey ? ghost_targets(j, a.Ny, a.bcy, ty + 1, fy + 1) : 0);
-      for (int b = 0; b < cy; ++b)
-        for (int c = 0; c < cx; ++c) {
-          if (b == 0 && c == 0) continue;
-          const long long gg = (long long)(ty[b] + HALO) * P + (tx[c] + HALO);
-          if (!gok(gg, PL)) continue;
-          Qd[gg] = q.r;
-          Qd[PL + gg] = fx[c] ? q.u * -1.0 : q.u;
-          Qd[2 * PL + gg] = fy[b] ? q.v * -1.0 : q.v;
-          Qd[3 * PL + gg] = q.p;
+      if constexpr (TX < 16) {
+        // a step of a small grid waits for these cells: no arrays in local
+        // memory (Sod 512 x 8 15.3 | 14.75 us a step; on full grids, which
+        // have other warps to run, the registers cost MUSCL-Hancock 1 %)
+        // which of the ghosts -2, -1, N, N + 1 of each axis copy this cell
+        unsigned xm = 0u, ym = 0u;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          bool flip;
+          if (ghost_source(t < 2 ? t - 2 : a.Nx + t - 2, a.Nx, a.bcx, &flip) == i) xm |= 1u << t;
+          if (ghost_source(t < 2 ? t - 2 : a.Ny + t - 2, a.Ny, a.bcy, &flip) == j) ym |= 1u << t;
         }
+        const bool fx = a.bcx == 1, fy = a.bcy == 1;  // reflecting
+#pragma unroll 1
+        for (unsigned mb = ym | 16u; mb; mb &= mb - 1u) {  // the ghost rows, then the cell's own
+          const int b = __ffs(mb) - 1;
+          const int ty = b == 4 ? j : b < 2 ? b - 2 : a.Ny + b - 2;
+          const double v = b < 4 && fy ? q.v * -1.0 : q.v;
+#pragma unroll 1
+          for (unsigned mc = b < 4 ? xm | 16u : xm; mc; mc &= mc - 1u) {
+            const int c = __ffs(mc) - 1;
+            const int tx = c == 4 ? i : c < 2 ? c - 2 : a.Nx + c - 2;
+            const long long gg = (long long)(ty + HALO) * P + (tx + HALO);
+            if (!gok(gg, PL)) continue;
+            Qd[gg] = q.r;
+            Qd[PL + gg] = c < 4 && fx ? q.u * -1.0 : q.u;
+            Qd[2 * PL + gg] = v;
+            Qd[3 * PL + gg] = q.p;
+          }
+        }
+      } else {
+        int tx[5], ty[5];
+        bool fx[5], fy[5];
+        tx[0] = i; fx[0] = false;
+        ty[0] = j; fy[0] = false;
+        const int cx = 1 + (ex ? ghost_targets(i, a.Nx, a.bcx, tx + 1, fx + 1) : 0);
+        const int cy = 1 + (ey ? ghost_targets(j, a.Ny, a.bcy, ty + 1, fy + 1) : 0);
+        for (int b = 0; b < cy; ++b)
+          for (int c = 0; c < cx; ++c) {
+            if (b == 0 && c == 0) continue;
+            const long long gg = (long long)(ty[b] + HALO) * P + (tx[c] + HALO);
+            if (!gok(gg, PL)) continue;
+            Qd[gg] = q.r;
+            Qd[PL + gg] = fx[c] ? q.u * -1.0 : q.u;
+            Qd[2 * PL + gg] = fy[b] ? q.v * -1.0 : q.v;
+            Qd[3 * PL + gg] = q.p;
+          }
+      }
     }
   }
 
