@@ -12,6 +12,7 @@ struct BatchCfg {
   const char *name;
   size_t smem;
   const void *fn;
+  bool by_name = false;  // runs when asked for (tile_config), no candidate of the autotuner
 };
 
 // The two-column march configurations (batch_march2.cu).

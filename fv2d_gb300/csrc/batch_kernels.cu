@@ -56,6 +56,8 @@ static const std::vector<BatchCfg> &all_cfgs() {
   return v;
 }
 
+bool batch_cfg_by_name(int i) { return all_cfgs()[i].by_name; }
+
 int batch_num_cfgs() { return (int)all_cfgs().size(); }
 
 void batch_cfg_info(int i, int *tx, int *ty, int *nt, int *staging, size_t *smem, const char **name, int *fams) {

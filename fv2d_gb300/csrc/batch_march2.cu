@@ -12,16 +12,17 @@ namespace fv2d {
 #define FV2D_MARCH2(H, NT, MINB, NAME) \
   {bm2::STRIP, H, NT, 2, 1 << FAM_PLAIN, NAME, 0, (const void *)batch_march2_kernel<NT, MINB, false>}
 #define FV2D_MARCH2_DIFF(H, NT, MINB, NAME) \
-  {bm2::STRIP, H, NT, 2, 1 << FAM_DIFF, NAME, 0, (const void *)batch_march2_kernel<NT, MINB, true>}
+  {bm2::STRIP, H, NT, 2, 1 << FAM_DIFF, NAME, 0, (const void *)batch_march2_kernel<NT, MINB, true>, true}
 
 static const BatchCfg kMarch2[] = {
     // named <strip columns>/<threads per CTA>x<CTAs per SM>/march2[-diff]
     FV2D_MARCH2(32, 32, 16, "60/32x16/march2"),
     FV2D_MARCH2(32, 32, 12, "60/32x12/march2"),
-    // the diffusive body: 16 CTAs per SM where the lane then runs in fewer
-    // waves (RT 1400^2, ms per 100 steps: 5.54 | 6.25 at 10), 10 elsewhere
-    // (RT 1024 x 3072 8.75 | 8.59, 128 x 384 1.22 | 1.19)
-    FV2D_MARCH2_DIFF(32, 32, 16, "60/32x16/march2-diff"),
+    // The diffusive body is faster than the one-column march (RT 512 x 1536 x 200
+    // 5.6 | 6.2 ms, RT 2048^2 x 100 10.7 | 12.2) but rounds otherwise, and a flow
+    // past its instability amplifies that: 3.5e-5 of the state between the two
+    // kernels after 200 steps of one such run.  A request's result must not depend
+    // on which of two close trials won at start-up, so it runs by name only.
     FV2D_MARCH2_DIFF(32, 32, 10, "60/32x10/march2-diff"),
 };
 

@@ -94,21 +94,21 @@ __device__ __forceinline__ void hll(const Q2 &qL, const Q2 &qR, Q2 &f, f2 &pout,
   const f2 SL = min2(qL.u - aL, qR.u - aR);
   const f2 SR = max2(qL.u + aL, qR.u + aR);
   const f2 peL = qL.p * g.entho, peR = qR.p * g.entho;
-  const f2 EL = fma2(g.half * qL.r, fma2(qL.u, qL.u, qL.v * qL.v), peL);
-  const f2 ER = fma2(g.half * qR.r, fma2(qR.u, qR.u, qR.v * qR.v), peR);
+  const f2 EL = peL + (g.half * qL.r) * fma2(qL.u, qL.u, qL.v * qL.v);
+  const f2 ER = peR + (g.half * qR.r) * fma2(qR.u, qR.u, qR.v * qR.v);
   const f2 ruL = qL.r * qL.u, ruR = qR.r * qR.u;
   const Q2 FL{ruL, fma2(ruL, qL.u, qL.p), ruL * qL.v, (qL.p + EL) * qL.u};
   const Q2 FR{ruR, fma2(ruR, qR.u, qR.p), ruR * qR.v, (qR.p + ER) * qR.u};
   const f2 mvL = qL.r * qL.v, mvR = qR.r * qR.v;
   const f2 uEL = fma2(g.half * fma2(ruL, ruL, mvL * mvL), rrL, peL);
   const f2 uER = fma2(g.half * fma2(ruR, ruR, mvR * mvR), rrR, peR);
-  const f2 SLSR = SL * SR, nSL = F2(0.f) - SL;
+  const f2 SLSR = SL * SR;
   const f2 rden = rcp2(SR - SL);
   Q2 FM;
-  FM.r = fma2(SLSR, qR.r - qL.r, fma2(SR, FL.r, nSL * FR.r)) * rden;
-  FM.u = fma2(SLSR, ruR - ruL, fma2(SR, FL.u, nSL * FR.u)) * rden;
-  FM.v = fma2(SLSR, mvR - mvL, fma2(SR, FL.v, nSL * FR.v)) * rden;
-  FM.p = fma2(SLSR, uER - uEL, fma2(SR, FL.p, nSL * FR.p)) * rden;
+  FM.r = fma2(SLSR, qR.r - qL.r, SR * FL.r - SL * FR.r) * rden;
+  FM.u = fma2(SLSR, ruR - ruL, SR * FL.u - SL * FR.u) * rden;
+  FM.v = fma2(SLSR, mvR - mvL, SR * FL.v - SL * FR.v) * rden;
+  FM.p = fma2(SLSR, uER - uEL, SR * FL.p - SL * FR.p) * rden;
   const f2 pM = g.half * (qL.p + qR.p);
   const b2 lf = ge0(SL), rt0 = le0(SR);
   const b2 rt{!lf.x && rt0.x, !lf.y && rt0.y};
@@ -328,7 +328,7 @@ __device__ __forceinline__ void march2_item(const BatchArgs &a, const WorkItem i
   // and the y face terms of row C, and row C - 1's velocities: half the
   // arithmetic, a third of the shuffles and none of the loads and conversions of
   // forming the four faces of each cell from its 3 x 3 neighbours (RT 1024 x
-  // 3072, HLL, ms per 100 steps: 9.38 | 8.6; the one-column march 8.9).
+  // 3072, HLL, ms per 100 steps: 9.38 | 8.14; the one-column march 8.9).
   struct V2 {
     f2 u, v;
   };

@@ -441,15 +441,17 @@ __device__ __forceinline__ void riemann_hll(const S4<double> &qL, const S4<doubl
 // RiemannSolvers.h:53-128.  The star state is evaluated once, for the side
 // the reference would pick if it reaches the star branches (uS > 0 -> left,
 // otherwise right), then the final state is chosen in the reference's order.
-// The side K is picked once (SL > 0 takes the left state whatever uS is), so
-// every select serves the star state and the flux, the total energy is formed
-// for that side only, and the larger sound speed is the root of the larger
-// square.
 template <class R>
 __device__ __forceinline__ void riemann_hllc(const S4<R> &qL, const S4<R> &qR, S4<R> &f, R &pout, const Gas<R> &g) {
   const R rL = qL.r, uL = qL.u, vL = qL.v, pL = qL.p;
   const R rR = qR.r, uR = qR.u, vR = qR.v, pR = qR.p;
-  const R cmax = dsqrt(fv_fmax(fv_div(pL * g.gamma, rL), fv_div(pR * g.gamma, rR)));
+  const R ekL = (fv_half(rL) * ((uL * uL) + (vL * vL)));
+  const R EL = ekL + (pL * g.entho);
+  const R ekR = (fv_half(rR) * ((uR * uR) + (vR * vR)));
+  const R ER = ekR + (pR * g.entho);
+  const R cL = sound_speed(qL, g);
+  const R cR = sound_speed(qR, g);
+  const R cmax = fv_fmax(cL, cR);
   const R SL = fv_fmin(uL, uR) - cmax;
   const R SR = fv_fmax(uL, uR) + cmax;
   const R rcL = (rL * (uL - SL));
@@ -457,26 +459,29 @@ __device__ __forceinline__ void riemann_hllc(const S4<R> &qL, const S4<R> &qR, S
   R uS, pS;
   fv_div2((rcR * uR) + (rcL * uL) + (pL - pR),
           (rcR * pL) + (rcL * pR) + ((rcL * rcR) * (uL - uR)), rcR + rcL, uS, pS);
-  // branch order of RiemannSolvers.h:89-112
-  const bool sideL = fv_gt0(uS), bL = fv_gt0(SL);
-  const bool left = bL || sideL;
-  const bool star = !bL && (sideL || fv_gt0(SR));
-  const R rK = left ? rL : rR;
-  const R uK = left ? uL : uR;
-  const R vK = left ? vL : vR;
-  const R pK = left ? pL : pR;
-  const R SK = left ? SL : SR;
-  const R EK = (fv_half(rK) * ((uK * uK) + (vK * vK))) + (pK * g.entho);
+  const bool sideL = fv_gt0(uS);
+  const R rK = sideL ? rL : rR;
+  const R uK = sideL ? uL : uR;
+  const R pK = sideL ? pL : pR;
+  const R EK = sideL ? EL : ER;
+  const R SK = sideL ? SL : SR;
   R rS, ES;
   fv_div2((rK * (SK - uK)), ((SK - uK) * EK) - (pK * uK) + (pS * uS), SK - uS, rS, ES);
-  const R sr = star ? rS : rK;
-  const R su = star ? uS : uK;
-  const R sp = star ? pS : pK;
-  const R E = star ? ES : EK;
+  // branch order of RiemannSolvers.h:89-112
+  const bool bL = fv_gt0(SL);
+  const bool bStar = !bL && (sideL || fv_gt0(SR));
+  R sr, su, sv, sp, E;
+  if (bL) {
+    sr = rL; su = uL; sv = vL; sp = pL; E = EL;
+  } else if (bStar) {
+    sr = rS; su = uS; sv = sideL ? vL : vR; sp = pS; E = ES;
+  } else {
+    sr = rR; su = uR; sv = vR; sp = pR; E = ER;
+  }
   pout = sp;
   f.r = (sr * su);
   f.u = ((sr * su) * su) + sp;
-  f.v = (f.r * vK);
+  f.v = (f.r * sv);
   f.p = ((E + sp) * su);
 }
 

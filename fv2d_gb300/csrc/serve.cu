@@ -42,6 +42,7 @@
 
 namespace fv2d {
 int batch_num_cfgs();
+bool batch_cfg_by_name(int i);
 void batch_cfg_info(int i, int *tx, int *ty, int *nt, int *staging, size_t *smem, const char **name, int *ext);
 cudaError_t batch_setup(int i, int *ctas_per_sm);
 cudaError_t batch_launch(int i, int grid, cudaStream_t s, const BatchArgs &a);
@@ -1234,7 +1235,8 @@ void autotune(fv2d_server *s) {
     double best = -1;
     int best_cfg = s->fam_cfg[f][kBuckets - 1];
     for (int c = 0; c < ncfg; ++c) {
-      if (!s->cfg_grid[c] || !((cfg_fams(c) >> f) & 1)) continue;  // the family's configurations
+      // the family's configurations
+      if (!s->cfg_grid[c] || !((cfg_fams(c) >> f) & 1) || batch_cfg_by_name(c)) continue;
       for (int b = 0; b < kBuckets; ++b) s->fam_cfg[f][b] = c;
       double cells = 0, time = 0;  // one request of each bucket
       bool ok = true;

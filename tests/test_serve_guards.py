@@ -86,7 +86,7 @@ def test_ghost_columns_of_any_width(gpu_lib, scheme, bcx):
                                             mu=f(1e-4)),
              "extended": dict(reconstruction=fv.MUSCL_HANCOCK)}[scheme]
     configs = {"plain": ["28/32x20/march", "60/32x16/march2"],
-               "diffusive": ["28/32x20/march", "60/32x16/march2-diff"], "extended": [None]}[scheme]
+               "diffusive": ["28/32x20/march", "60/32x10/march2-diff"], "extended": [None]}[scheme]
     runs = []
     for nx in (16, 17, 27, 28, 29, 59, 60, 61, 62, 120, 121):
         for bcy, ny, ts in ((fv.BC_REFLECTING, 16, fv.TS_EULER), (fv.BC_PERIODIC, 19, fv.TS_RK2),
