@@ -118,12 +118,14 @@ __device__ __forceinline__ T sim_get(const WarpSim &s) {
 }
 #define FV2D_SIM(ws, field) bm::sim_get<decltype(SimDev::field), offsetof(SimDev, field)>(ws)
 
-// The ghost columns that copy a lane's column or pair of columns
-// (BoundaryConditions.h:82-147, inverse map): at most two for the 16 or more
-// columns a request has.  They are found once per work item: the warps of the
-// outer strips write them in every row, and a step of one or two waves ends when
-// those warps do (finding them row by row cost such lanes 4 to 9 %).  Packed
-// into a word (15 bits a column), for the registers.
+// The ghost columns that copy a pair of columns (BoundaryConditions.h:82-147,
+// inverse map), for the two-column march: at most two for the 16 or more columns
+// a request has.  They are found once per work item: the warps of the outer
+// strips write them in every row, and a step of one or two waves ends when those
+// warps do (finding them row by row, through arrays in local memory, cost such
+// lanes 4 to 9 %).  Packed into a word (15 bits a column), for the registers; the
+// one-column march has none to spare at 20 warps per SM (RT 1024 x 3072 x 100:
+// 8.96 ms row by row, 9.86 once per item) and finds them row by row.
 struct XGhosts {
   unsigned w;
   __device__ __forceinline__ bool any() const { return w != 0u; }
@@ -255,18 +257,21 @@ __device__ __forceinline__ void march_item(const BatchArgs &a, const WorkItem it
   const int ntiles = FV2D_SIM(W, ntx) * FV2D_SIM(W, nty);
   const int Nx = S.Nx, Ny = S.Ny;
   const int gxl = item.tx * STRIP + lane;           // padded column of this lane
-  const int gld = min(gxl, Nx + 3);                 // past the row's end: its last column, which reaches no output
+  const bool colok = gxl < Nx + 4;
   const bool out_lane = lane >= 2 && lane < 30 && gxl - 2 < Nx;
-  const XGhosts xg = out_lane ? x_ghosts(gxl - 2, false, Nx, S.bcx) : XGhosts{0u};
   const int band = FV2D_SIM(W, band);
   const int j0 = item.ty * band, jend = min(j0 + band, Ny);  // interior rows [j0, jend)
   const float dtdx = S.dt * S.inv_dx, dtdy = S.dt * S.inv_dy;
   const float ax = 0.5f * S.dt * S.inv_dx, ay = 0.5f * S.dt * S.inv_dy;  // MUSCL-Hancock half step
 
   auto load = [&](int L, float u[4]) {  // padded row L
-    const long long g = (long long)L * S.P + gld;
+    const long long g = (long long)L * S.P + gxl;
+    if (colok) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) u[k] = __ldg(S.src + k * S.PL + g);
+      for (int k = 0; k < 4; ++k) u[k] = __ldg(S.src + k * S.PL + g);
+    } else {
+      u[0] = 1.f; u[1] = 0.f; u[2] = 0.f; u[3] = 1.f;  // never reaches an output lane
+    }
   };
   const S4<float> zero4{0.f, 0.f, 0.f, 0.f};
   // y slopes from the row differences D(row) = q(row) - q(row - 1)
@@ -446,6 +451,7 @@ __device__ __forceinline__ void march_item(const BatchArgs &a, const WorkItem it
       }
 
       if (out_lane) {
+        const int i = gxl - 2;
         const long long g = (long long)C * S.P + gxl;
         if (S.avg) {  // SSP-RK2: 0.5 (U^n + U**) (Update.h:214-220), offsets alike
   #pragma unroll
@@ -454,45 +460,37 @@ __device__ __forceinline__ void march_item(const BatchArgs &a, const WorkItem it
   #pragma unroll
         for (int k = 0; k < 4; ++k) S.dst[k * S.PL + g] = un[k];
         if (S.last) {
-          // primitive state of the new cell for the next dt; the negative and
-          // NaN guards leave the common path through one test
-          const float r = un[0] + S.bg_r, rr = __fdividef(1.f, r);
-          const float u = __fmul_rn(un[1], rr), v = __fmul_rn(un[2], rr);
-          const float p = pressure_of(un[3], S.bg_e, r, u, v, S.gm1, S.lowmach);
-          float cs2 = __fmul_rn(__fmul_rn(p, S.gamma), rr);
-          if (!(min_nan(r, p) >= 0.f)) {  // a NaN of any field reaches the pressure
-            nnan += is_nan_f(p);
-            nneg += (r < 0.f) + (p < 0.f);
-            cs2 = (p < 0.f ? 1e-8f : p) * S.gamma / (r < 0.f ? 1e-8f : r);
-          }
-          const float cs = sqrtf(cs2);
+          // primitive state of the new cell for the next dt, negative guard
+          float r = un[0] + S.bg_r, u = un[1] / r, v = un[2] / r;
+          float p = pressure_of(un[3], S.bg_e, r, u, v, S.gm1, S.lowmach);
+          nnan += is_nan_f(r) | is_nan_f(u) | is_nan_f(v) | is_nan_f(p);
+          nneg += (r < 0.f) + (p < 0.f);
+          if (r < 0.f) r = 1e-8f;
+          if (p < 0.f) p = 1e-8f;
+          const float cs = sqrtf(p * S.gamma / r);
           const float ih = (cs + fabsf(u)) * S.inv_dx + (cs + fabsf(v)) * S.inv_dy;
-          lmax = fmaxf(lmax, ih);  // NaN never enters
+          if (ih > lmax) lmax = ih;  // NaN never enters
         } else {
-          nnan += is_nan_f(min_nan(min_nan(un[0], un[1]), min_nan(un[2], un[3])));
+          nnan += is_nan_f(un[0]) | is_nan_f(un[1]) | is_nan_f(un[2]) | is_nan_f(un[3]);
         }
-        // ghost copies (BoundaryConditions.h:82-147, inverse map): the cell's
-        // row, then, for rows whose ghosts copy it, each of those rows
-        const bool ey = j < 2 || j >= Ny - 2;
-        if (ey || xg.any()) {
-#pragma unroll 1
-          for (int t = ey ? 0 : 4; t < 5; ++t) {
-            int ty = j;
-            bool flip = false;
-            if (t < 4) {
-              ty = t < 2 ? t - 2 : Ny + t - 2;
-              if (ghost_source(ty, Ny, S.bcy, &flip) != j) continue;
+        // ghost copies (BoundaryConditions.h:82-147, inverse map)
+        const bool ex = (i < 2 || i >= Nx - 2), ey = (j < 2 || j >= Ny - 2);
+        if (ex || ey) {
+          int tx[5], ty[5];
+          bool nx[5], ny[5];
+          tx[0] = i; nx[0] = false;
+          ty[0] = j; ny[0] = false;
+          const int cx = 1 + (ex ? ghost_targets(i, Nx, S.bcx, tx + 1, nx + 1) : 0);
+          const int cy = 1 + (ey ? ghost_targets(j, Ny, S.bcy, ty + 1, ny + 1) : 0);
+          for (int b = 0; b < cy; ++b)
+            for (int c = 0; c < cx; ++c) {
+              if (b == 0 && c == 0) continue;
+              const long long gg = (long long)(ty[b] + 2) * S.P + (tx[c] + 2);
+              S.dst[gg] = un[0];
+              S.dst[S.PL + gg] = nx[c] ? -un[1] : un[1];
+              S.dst[2 * S.PL + gg] = ny[b] ? -un[2] : un[2];
+              S.dst[3 * S.PL + gg] = un[3];
             }
-            float *row = S.dst + (long long)(ty + 2) * S.P;
-#pragma unroll
-            for (int k = 0; k < 4; ++k, row += S.PL) {
-              const float x = k == 2 && flip ? -un[k] : un[k];
-              if (t < 4) row[gxl] = x;
-              const float xx = k == 1 && S.bcx == 1 ? -x : x;  // reflecting
-              if (xg.any()) row[xg.a()] = xx;
-              if (xg.two()) row[xg.b()] = xx;
-            }
-          }
         }
       }
 
