@@ -300,8 +300,8 @@ __device__ __forceinline__ void march2_item(const BatchArgs &a, const WorkItem i
   // conservative.
   // The loop is bound by instruction issue and by the latency of its chain at 16
   // warps per SM, so rare work (negative or NaN cells, the low-Mach recovery)
-  // leaves it through one branch at each end: KH 2048^2, PLM + HLLC, 49.0 G
-  // cell-updates/s with a select for each case, 56.3 G now.
+  // leaves it through one branch at each end, HLLC picks its side once and loads
+  // need no column test: KH 2048^2 x 200, PLM + HLLC, 17.1 | 14.9 ms.
   // The window carries the primitives of rows L - 2 and L - 1 (q0, qp), the
   // y slope of row L - 2, the y flux of face C - 1/2 and the prefetched next
   // row; the conservative row C is read again at its update (an L1 hit: it

@@ -74,8 +74,8 @@ __device__ __forceinline__ double div_spacing(double x, double d, double inv_d, 
 // cell): each thread takes the binary32 upper bound (physics.cuh) of its 16
 // cells from one pass over them, and only the cells whose bound is within the
 // bounds' slack of the CTA's largest are evaluated exactly (a second read,
-// from L2).  Evaluating every cell exactly took 109 us,
-// against 28 us of HBM time.
+// from L2).  Evaluating every cell exactly took 109 us
+// at 3000 x 2000, this 45, against 28 us of HBM time.
 __global__ void __launch_bounds__(kThreads) dt_noalloc_kernel(DtArgs a) {
   __shared__ double red[kThreads / 32];
   __shared__ float redf[kThreads / 32];

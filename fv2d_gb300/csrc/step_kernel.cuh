@@ -19,9 +19,10 @@
 //      cell that copies it (BoundaryConditions.h:82-147, inverse map), and
 //      folds the next step's inverse hyperbolic dt (ComputeDt.h:26-52) into a
 //      warp-shuffle max and one atomic per CTA;
-//   6. a one-thread kernel that follows in stream order commits t += dt, the
-//      counters and the next dt, and evaluates the device-driven loop
-//      condition (main.cpp:62-64); the step's CTAs only fire their reduction
+//   6. t += dt, the counters, the next dt and the device-driven loop condition
+//      (main.cpp:62-64) are committed by a one-thread kernel that follows in
+//      stream order, or, in the device loops of small grids, by every CTA of the
+//      next step for itself (Clock); the step's CTAs only fire their reduction
 //      atomics and exit (no fence, no last-CTA election).
 // Built with -fmad=false the results are bit-identical to the reference's
 // binary64 arithmetic.
