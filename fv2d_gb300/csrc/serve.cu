@@ -545,7 +545,10 @@ bool reserve_work(fv2d_server *s, int b, int need) {
 }
 
 // Admit one request into a free slot; returns the slot, or -1 when it does
-// not fit (HBM budget, table or work-list capacity).
+// not fit (HBM budget, table or work-list capacity).  The worker's stream must
+// hold no work on the table by now: the set-up runs on the admission streams,
+// ordered before what that stream is given next (join_admissions), not after
+// what it still holds.
 int admit(fv2d_server *s, const Pending &pd) {
   const NvtxRange nvtx_range("fv2d_server admit");
   if (s->free_slots.empty()) return -1;
@@ -1202,7 +1205,10 @@ double autotune_trial(fv2d_server *s, int family, int Nx, int Ny, int nsims) {
       s->h_up[k].status = SIM_FREE;
       s->free_slots.push_back(k);
     }
+  // the next trial's requests are set up on the admission streams, which wait
+  // for nothing on this one, and from the same table (admit)
   cudaMemcpyAsync(s->d_sims, s->h_up, sizeof(SimDev) * s->max_sims, cudaMemcpyHostToDevice, s->stream);
+  cudaStreamSynchronize(s->stream);
   s->n_admitted = 0;
   s->n_active = 0;
   for (int q = 0; q < kLanes; ++q) s->items_in[q] = 0;
