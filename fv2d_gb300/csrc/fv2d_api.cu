@@ -106,17 +106,38 @@ bool is_pow2_spacing(double d) {
   return m == 0.5 && std::isfinite(1.0 / d);
 }
 
+// A driver function by name (null where the driver has none).
+template <class F>
+F driver_entry(const char *name) {
+  void *ptr = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  if (cudaGetDriverEntryPointByVersion(name, &ptr, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+      q != cudaDriverEntryPointSuccess)
+    return nullptr;
+  return reinterpret_cast<F>(ptr);
+}
 PFN_cuTensorMapEncodeTiled_v12000 get_encode() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  if (!fn) {
-    void *ptr = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &ptr, 12000, cudaEnableDefault, &q) ==
-            cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(ptr);
-  }
+  static const auto fn = driver_entry<PFN_cuTensorMapEncodeTiled_v12000>("cuTensorMapEncodeTiled");
   return fn;
+}
+
+// Whether a kernel of the context may read or write the `bytes` at p itself:
+// binary64 words in one allocation of the context's device.  Any other array
+// (on another device, managed or host memory, a range that leaves its
+// allocation, no address of the driver's at all) takes the runtime's copy,
+// which moves it or returns an error where a kernel would fault.
+bool usable_in_place(const fv2d_ctx *c, const double *p, size_t bytes) {
+  static const auto range = driver_entry<PFN_cuMemGetAddressRange_v3020>("cuMemGetAddressRange");
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+  if (at.type != cudaMemoryTypeDevice || at.device != c->device || a % sizeof(double) || !range) return false;
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  return range(&base, &size, (CUdeviceptr)a) == CUDA_SUCCESS && a - base <= size && bytes <= size - (a - base);
 }
 
 // ------------------------------------------------------------------ kernels
@@ -639,11 +660,16 @@ int fv2d_set_stream(fv2d_ctx *ctx, void *stream) {
 
 int fv2d_set_prim_device(fv2d_ctx *ctx, const double *q_dev) {
   if (!ctx || !q_dev) return FV2D_ERR_INVALID;
-  // the set-up kernel reads the caller's array itself (a copy to the staging
-  // buffer first moved 64 B a cell more: 4096^2 0.16 ms); a prefetch that was
-  // waiting in that buffer is dropped, as by any new state
+  // the set-up kernel reads the caller's array itself where it may (a copy to
+  // the staging buffer first moves 64 B a cell more: 4096^2 0.16 ms); a prefetch
+  // that was waiting in that buffer is dropped, as by any new state
+  const size_t bytes = (size_t)ctx->p.Nx * ctx->p.Ny * 4 * sizeof(double);
   stage_take(ctx);
-  return run_prepare(ctx, q_dev);
+  if (usable_in_place(ctx, q_dev, bytes)) return run_prepare(ctx, q_dev);
+  CK(cudaMemcpyAsync(ctx->stage, q_dev, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+  const int rc = run_prepare(ctx, ctx->stage);
+  stage_release(ctx);
+  return rc;
 }
 
 int fv2d_set_prim(fv2d_ctx *ctx, const double *q_host) {
@@ -728,7 +754,8 @@ int fv2d_init_problem(fv2d_ctx *ctx, int problem) {
 static int get_planes(fv2d_ctx *ctx, const double *planes, double *dst, cudaMemcpyKind kind) {
   const fv2d_params &p = ctx->p;
   const long long n = (long long)p.Nx * p.Ny;
-  if (kind == cudaMemcpyDeviceToDevice) {  // straight into the caller's array
+  const size_t bytes = (size_t)n * 4 * sizeof(double);
+  if (kind == cudaMemcpyDeviceToDevice && usable_in_place(ctx, dst, bytes)) {  // straight into the caller's array
     pack_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(planes, ctx->plane, ctx->pitch, p.Nx, p.Ny, dst);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(ctx->stream));
@@ -738,7 +765,7 @@ static int get_planes(fv2d_ctx *ctx, const double *planes, double *dst, cudaMemc
   pack_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(planes, ctx->plane, ctx->pitch, p.Nx, p.Ny,
                                                                      ctx->stage);
   CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(dst, ctx->stage, (size_t)n * 4 * sizeof(double), kind, ctx->stream));
+  CK(cudaMemcpyAsync(dst, ctx->stage, bytes, kind, ctx->stream));
   stage_release(ctx);
   CK(cudaStreamSynchronize(ctx->stream));
   return FV2D_OK;

@@ -82,8 +82,9 @@ int fv2d_get_prim(fv2d_ctx *ctx, double *q_host);
  * reading the host link.  q_host must not change between the two calls.  Any
  * other use of the staging buffer in between (fv2d_set_prim with another
  * pageable array, fv2d_set_prim_device, fv2d_init_problem, fv2d_get_prim
- * other than of the host mirror, fv2d_get_cons) waits for the copy and drops
- * it; fv2d_set_prim then reads q_host again.  FV2D_ERR_INVALID for pageable
+ * other than of the host mirror, fv2d_get_prim_device into an array it cannot
+ * write in place, fv2d_get_cons) waits for the copy and drops it;
+ * fv2d_set_prim then reads q_host again.  FV2D_ERR_INVALID for pageable
  * memory. */
 int fv2d_prefetch_prim(fv2d_ctx *ctx, const double *q_host);
 
@@ -99,10 +100,12 @@ int fv2d_set_host_mirror(fv2d_ctx *ctx, double *q_host);
 int fv2d_get_cons(fv2d_ctx *ctx, double *u_host);
 
 /* Same as set_prim / get_prim with device-resident interleaved arrays.
- * set_prim_device is ordered on the context's stream and returns before the
- * copy has run: q_dev must not change until work on that stream after the
- * call (or a synchronisation) has completed.  get_prim_device returns with the
- * copy complete. */
+ * Arrays in one allocation of the context's device are read and written in
+ * place; any other (on another device, managed) is copied by the runtime, which
+ * refuses what it cannot reach (FV2D_ERR_CUDA).  set_prim_device is ordered on
+ * the context's stream and returns before the array has been read: q_dev must
+ * not change until work on that stream after the call (or a synchronisation) has
+ * completed.  get_prim_device returns with the array complete. */
 int fv2d_set_prim_device(fv2d_ctx *ctx, const double *q_dev);
 int fv2d_get_prim_device(fv2d_ctx *ctx, double *q_dev);
 
