@@ -157,6 +157,10 @@ class BufferPool {
     held_ += bytes;
     free_.push_back(std::move(b));
   }
+  size_t kept() {  // bytes
+    std::lock_guard<std::mutex> lock(mu_);
+    return held_;
+  }
 
  private:
   std::mutex mu_;
