@@ -141,7 +141,11 @@ __host__ __device__ __forceinline__ bool fv_isnan(float x) { return isnan(x); }
 // HLLC: 4 1.02 | 1.07, 6 1.02 | 1.06, 7 1.05 | 1.06; its PCM form: 5 0.80 | 0.77;
 // HLL: 9 1.58 | 1.40; FSLP RK2 777 x 1501: 3 0.327 | 0.334 a stage; RT
 // 1024 x 3072: 10 1.64 | 1.60, 12 1.48 | 1.46.
-constexpr int kSoftMulHllc = 31127, kSoftMul = kSoftMulHllc & ~4, kSoftMulVisc = kSoftMul | 512;
+template <int... GROUPS>
+constexpr int soft_groups = ((1 << (GROUPS - 1)) | ...);
+constexpr int kSoftMulHllc = soft_groups<1, 2, 3, 5, 8, 9, 12, 13, 14, 15>;
+constexpr int kSoftMul = soft_groups<1, 2, 5, 8, 9, 12, 13, 14, 15>;          // HLL and FSLP
+constexpr int kSoftMulVisc = soft_groups<1, 2, 5, 8, 9, 10, 12, 13, 14, 15>;  // the same with viscosity
 // Sums and differences.  In binary64 on the device a + b is issued as the
 // multiply-add a * one + b, with `one` = 1 in a register that the compiler
 // cannot see through: the same correctly rounded sum (signed zeros, infinities
@@ -206,10 +210,6 @@ __host__ __device__ __forceinline__ void fv_quot2(double a1, double b1, double a
   q2 = a2 / b2;
 #endif
 }
-__host__ __device__ __forceinline__ void fv_quot2(float a1, float b1, float a2, float b2, float &q1, float &q2) {
-  q1 = a1 / b1;
-  q2 = a2 / b2;
-}
 __host__ __device__ __forceinline__ void fv_div2_by(double a1, double a2, double b, uint32_t r, double &q1, double &q2) {
 #ifdef __CUDA_ARCH__
   const double2 q = softfp::div2_by(a1, a2, b, r);
@@ -220,10 +220,6 @@ __host__ __device__ __forceinline__ void fv_div2_by(double a1, double a2, double
   q1 = a1 / b;
   q2 = a2 / b;
 #endif
-}
-__host__ __device__ __forceinline__ void fv_div2_by(float a1, float a2, float b, uint32_t, float &q1, float &q2) {
-  q1 = a1 / b;
-  q2 = a2 / b;
 }
 
 enum { IR = 0, IU = 1, IV = 2, IP = 3, IE = 3 };
