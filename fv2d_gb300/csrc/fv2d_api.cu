@@ -37,6 +37,7 @@ using namespace fv2d;
 struct fv2d_ctx {
   fv2d_params p;
   int device = 0;
+  int sms = 0;  // the device's SM count
   cudaStream_t own_stream = nullptr, stream = nullptr;
   int tile = TILE_WIDE;  // TILE_* of the step (choose_tile)
   int pitch = 0;
@@ -298,9 +299,9 @@ dim3 grid_of(const fv2d_params &p) {
 // at about three to an SM (us a step, wide | small: Sod 512 x 8, 64 small
 // tiles, 27 | 18; KH 64^2, 64, 33 | 25; 128^2, 256, 33 | 27; 192^2, 576,
 // 35 | 34; 256^2, 1024, 40 | 52).
-int choose_tile(const fv2d_params &p) {
+int choose_tile(const fv2d_params &p, int sms) {
   const dim3 g = grid_of<SmallTile>(p);
-  return (long long)g.x * g.y <= 3 * 152 ? TILE_SMALL : TILE_WIDE;
+  return (long long)g.x * g.y <= 3 * sms ? TILE_SMALL : TILE_WIDE;
 }
 dim3 tile_grid(const fv2d_ctx *c) {
   return c->tile == TILE_SMALL ? grid_of<SmallTile>(c->p) : grid_of<WideTile>(c->p);
@@ -407,7 +408,7 @@ int launch_driven(fv2d_ctx *ctx, int n) {
   a.driven = 1;
   a.mirror = nullptr;  // device loops never write it
   a.chained = a.nblocks <= kChainedCtas;
-  a.overlapped = a.chained && (ctx->tile == TILE_SMALL ? a.nblocks <= 2 * 152 : a.nblocks > 3 * 152);
+  a.overlapped = a.chained && (ctx->tile == TILE_SMALL ? a.nblocks <= 2 * ctx->sms : a.nblocks > 3 * ctx->sms);
   for (int k = 0; k < n; ++k) {
     a.step = k;
     if (int rc = launch_stages(ctx, a)) return rc;
@@ -444,7 +445,7 @@ int run_prepare(fv2d_ctx *ctx, const double *src) {
   pa.Nx = p.Nx;
   pa.Ny = p.Ny;
   const long long n = (long long)p.Nx * p.Ny + 4LL * (p.Nx + 4) + 4LL * p.Ny;
-  const int nb = (int)std::min<long long>((n + 255) / 256, 8LL * 152);
+  const int nb = (int)std::min<long long>((n + 255) / 256, 8LL * ctx->sms);
   pa.nblocks = nb;
   pa.gamma = ctx->args.gamma;
   pa.gm1 = ctx->args.gm1;
@@ -573,6 +574,8 @@ int fv2d_create(const fv2d_params *p, int device, fv2d_ctx **out) {
     if ((e = cudaSetDevice(device)) != cudaSuccess) return bail(cuda_fail(ctx, e, "cudaSetDevice"));
   }
   cudaGetDevice(&ctx->device);
+  if ((e = cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->device)) != cudaSuccess)
+    return bail(cuda_fail(ctx, e, "cudaDeviceGetAttribute"));
   if ((e = init_step_kernels()) != cudaSuccess) return bail(cuda_fail(ctx, e, "step kernel attributes"));
   if ((e = cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking)) != cudaSuccess ||
       (e = cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking)) != cudaSuccess ||
@@ -581,7 +584,7 @@ int fv2d_create(const fv2d_params *p, int device, fv2d_ctx **out) {
     return bail(cuda_fail(ctx, e, "cudaStreamCreate"));
   ctx->stream = ctx->own_stream;
 
-  ctx->tile = choose_tile(*p);
+  ctx->tile = choose_tile(*p, ctx->sms);
   const int W = p->Nx + 4, H = p->Ny + 4;
   ctx->pitch = (W + 31) / 32 * 32;
   ctx->plane = (long long)H * ctx->pitch;

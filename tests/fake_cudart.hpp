@@ -42,7 +42,8 @@ struct Access {
 struct Launch {
   std::string kernel;
   cudaStream_t stream;
-  void *word;  // first word of the first argument
+  void *word;        // first word of the first argument
+  bool programmatic;  // may start before the previous launch has ended
 };
 struct Copy {
   const void *dst, *src;
@@ -63,6 +64,7 @@ struct Runtime {
   std::function<cudaPointerAttributes(const void *)> attributes;
   std::function<CUresult(CUdeviceptr *, size_t *, CUdeviceptr)> range;
   cudaError_t last = cudaSuccess;
+  int sms = 152;
 
   static void merge(VectorClock &a, const VectorClock &b) {
     for (auto &[s, t] : b) a[s] = std::max(a[s], t);
@@ -96,12 +98,12 @@ inline Runtime &rt() {
 }
 inline int id(const void *handle) { return (int)reinterpret_cast<uintptr_t>(handle); }
 
-inline void launch(const void *fn, void **args, cudaStream_t st) {
+inline void launch(const void *fn, void **args, cudaStream_t st, bool programmatic = false) {
   std::lock_guard<std::mutex> lock(rt().mu);
   rt().tick(id(st));
   void *word = nullptr;
   if (args && args[0]) std::memcpy(&word, args[0], sizeof word);
-  rt().launches.push_back({rt().names[fn], st, word});
+  rt().launches.push_back({rt().names[fn], st, word, programmatic});
 }
 inline CUresult encode_tiled(CUtensorMap *map, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                              const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
@@ -177,7 +179,11 @@ cudaError_t cudaLaunchKernel(const void *fn, dim3, dim3, void **args, size_t, cu
   return cudaSuccess;
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *fn, void **args) {
-  fake::launch(fn, args, c->stream);
+  bool programmatic = false;
+  for (unsigned k = 0; k < c->numAttrs; ++k)
+    programmatic |= c->attrs[k].id == cudaLaunchAttributeProgrammaticStreamSerialization &&
+                    c->attrs[k].val.programmaticStreamSerializationAllowed;
+  fake::launch(fn, args, c->stream, programmatic);
   return cudaSuccess;
 }
 cudaError_t cudaFuncSetAttribute(const void *, cudaFuncAttribute, int) { return cudaSuccess; }
@@ -193,7 +199,7 @@ cudaError_t cudaGetDevice(int *d) {
   return cudaSuccess;
 }
 cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr a, int) {
-  *v = a == cudaDevAttrMultiProcessorCount ? 152 : 1 << 20;
+  *v = a == cudaDevAttrMultiProcessorCount ? fake::rt().sms : 1 << 20;
   return cudaSuccess;
 }
 cudaError_t cudaGetLastError() {
