@@ -741,8 +741,8 @@ def main():
                      "traffic": (traffic * cells) if traffic else None, "peak_kind": peak_kind,
                      "bytes_per_cell": BYTES_PER_CELL, "kernel": "fv2d::step_kernel<PLM,HLLC>",
                      "duration": "CUDA events per iteration: the step kernel plus its one-thread commit kernel "
-                                 "(~4.7 us, 0.4 % of the iteration in the ncu launch list)",
-                     "binding": "instruction issue, not HBM: binary64 pipe ~64 %, integer ALU ~55 % busy "
+                                 "(~3.7 us, 0.4 % of the iteration in the ncu launch list)",
+                     "binding": "the binary64 pipe, not HBM: that pipe 80 %, integer ALU 50 % busy "
                                 "(profiles/step_fp64_plm_hllc_sedov.txt); see roofline_fp64"},
         "roofline_fp64": fp64,
         "cpu_baseline": cpu, "e2e": e2e, "clocks": clocks,

@@ -18,11 +18,13 @@ static const BatchCfg kMarch2[] = {
     // named <strip columns>/<threads per CTA>x<CTAs per SM>/march2[-diff]
     FV2D_MARCH2(32, 32, 16, "60/32x16/march2"),
     FV2D_MARCH2(32, 32, 12, "60/32x12/march2"),
-    // The diffusive body is faster than the one-column march (RT 512 x 1536 x 200
-    // 5.6 | 6.2 ms, RT 2048^2 x 100 10.7 | 12.2) but rounds otherwise, and a flow
-    // past its instability amplifies that: 3.5e-5 of the state between the two
-    // kernels after 200 steps of one such run.  A request's result must not depend
-    // on which of two close trials won at start-up, so it runs by name only.
+    // Unused unless asked for by name: diffusive requests keep the one-column
+    // march and its rounding.  This body is faster (RT 512 x 1536 x 200 5.6 | 6.2
+    // ms, RT 2048^2 x 100 10.7 | 12.2) but rounds otherwise, and a flow past its
+    // instability amplifies that: 3.5e-5 of the state between the two kernels
+    // after 200 steps of one such run.  (The plain family's two marches round
+    // differently as well; there the trials choose, and the two-column one wins
+    // them at every start: autotune.)
     FV2D_MARCH2_DIFF(32, 32, 10, "60/32x10/march2-diff"),
 };
 

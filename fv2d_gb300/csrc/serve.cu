@@ -1230,10 +1230,11 @@ double autotune_trial(fv2d_server *s, int family, int Nx, int Ny, int nsims) {
 // kernel alone, and per-bucket choices from short trials changed from one
 // start to the next.  The trials run under the service's own scheduling cap
 // (active_cells), so a configuration is measured at the load its lanes will
-// carry: on the 512-request stream at 8e6 cells per step the one-column march
-// (smaller work items, more resident warps) gave p50 0.089 s against 0.103 s
-// for the two-column one, which wins on full lanes (the same stream submitted
-// at once: 50.1 against 48.9 G cell-updates/s).
+// carry.  For the plain family they are not close: 12 starts of 12 took the
+// two-column march (six at 8e6 cells per step, six without a cap), which gives
+// the 512-request stream p50 0.038 s against the one-column march's 0.075 and,
+// submitted at once under the cap, 55.9 against 46.8 G cell-updates/s.
+// Configurations marked by_name are not tried.
 void autotune(fv2d_server *s) {
   const int rep[kBuckets] = {96, 192, 384, 768};
   const int ncfg = num_cfgs();
