@@ -1,4 +1,5 @@
 """Builds a host harness from the library's objects and fake_cudart.hpp."""
+import glob
 import os
 import shutil
 import subprocess
@@ -17,8 +18,12 @@ def build_with_fake_runtime(tmp_path, harness):
         nvcc = b._nvcc()
     except RuntimeError:
         return None
-    include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
-    if not cxx or not os.path.exists(os.path.join(include, "cuda_runtime_api.h")):
+    roots = [os.environ.get("CUDA_HOME", ""), *(os.path.dirname(os.path.dirname(f(nvcc)))
+                                                for f in (os.path.abspath, os.path.realpath)), "/usr/local/cuda"]
+    include = next((d for r in roots for d in [os.path.join(r, "include"),
+                                               *glob.glob(os.path.join(r, "targets", "*", "include"))]
+                    if os.path.exists(os.path.join(d, "cuda_runtime_api.h"))), None)
+    if not cxx or not include:
         return None
     b.build()
     exe = str(tmp_path / "harness")
